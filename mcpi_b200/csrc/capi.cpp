@@ -10,6 +10,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -194,6 +195,38 @@ std::vector<cplx> pack_momentum(const std::vector<cplx> &Ht, int P, int M)
     return out;
 }
 
+// Outer-product factors of a momentum-block pair matrix (layout in kernels.h,
+// PairOp::contact): u[P] | w[P] with Ht[a][b] = u_a w_b inside every block,
+// all real. Each block's row and column through its largest entry give the
+// factors; empty when some value is complex or differs from its product by
+// more than rounding (4 ulp: the same values up to the order of multiplication).
+std::vector<double> pack_contact(const std::vector<cplx> &Ht, int P, int M)
+{
+    std::vector<double> f(2 * (size_t)P, 0.0);
+    for (int K = 0; K <= 2 * M - 2; ++K) {
+        const int qlo = K - (M - 1) > 0 ? K - (M - 1) : 0, n = K / 2 - qlo + 1;
+        auto pr = [&](int r) { return mcpi::pair_index(qlo + r, K - qlo - r, M); };
+        auto at = [&](int r, int c) { return Ht[(size_t)pr(r) * P + pr(c)]; };
+        int pr0 = 0, pc0 = 0;
+        for (int r = 0; r < n; ++r)
+            for (int c = 0; c < n; ++c) {
+                if (at(r, c).imag() != 0.0 || !std::isfinite(at(r, c).real())) return {};
+                if (std::fabs(at(r, c).real()) > std::fabs(at(pr0, pc0).real())) pr0 = r, pc0 = c;
+            }
+        const double piv = at(pr0, pc0).real();
+        for (int r = 0; r < n; ++r) {
+            f[pr(r)] = piv != 0.0 ? at(r, pc0).real() / piv : 0.0;
+            f[(size_t)P + pr(r)] = at(pr0, r).real();
+        }
+        for (int r = 0; r < n; ++r)
+            for (int c = 0; c < n; ++c) {
+                const double h = at(r, c).real();
+                if (!(std::fabs(f[pr(r)] * f[(size_t)P + pr(c)] - h) <= 8.9e-16 * std::fabs(h))) return {};
+            }
+    }
+    return f;
+}
+
 int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, const cplx *hdiag,
               const cplx *hfull)
 {
@@ -232,6 +265,7 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
         op.nhblk = (int)mom.size();
         op.hblk_h.resize(mom.size());
         std::memcpy(op.hblk_h.data(), mom.data(), sizeof(double2) * mom.size());
+        op.contact = pack_contact(Ht, P, M);
     }
     const std::vector<int> prog = pack_blocks(Ht, P, M);
     if (!prog.empty() && !sp->dense_only) {
@@ -253,29 +287,138 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
 }
 
 // A grow-only device buffer of the space: reused when large enough, else replaced.
-int reserve(void *&ptr, size_t &cap, size_t bytes)
-{
-    if (cap >= bytes && ptr) return MCPI_OK;
-    cudaFree(ptr);
-    ptr = nullptr;
-    cap = 0;
-    CK(cudaMalloc(&ptr, bytes ? bytes : 1));
-    cap = bytes;
-    return MCPI_OK;
-}
+int reserve(mcpi_space_s *sp, void *&ptr, size_t &cap, size_t bytes);
 
 int ensure_fused(mcpi_space_s *sp);
 
 PairOp op_view(const mcpi_space_s *sp, const DevPairOp &op);
 
-// The pair-space intermediate E (P x NC(N-2,M)) that the two-kernel and fused
-// forms of op pass between their halves; the direct form needs none.
-int ensure_E(mcpi_space_s *sp, const DevPairOp &op)
+size_t contact_bytes(const mcpi_space_s *sp)
+{
+    return sizeof(double2) * (size_t)(2 * sp->M - 1) * (size_t)sp->nc2;
+}
+
+// Stream-ordered scratch of the contact form on spaces whose calls the direct
+// form, which has no scratch, can take: each call allocates its S and gives it
+// back on its own stream, so calls on several streams or threads stay
+// independent, and a call that finds no memory runs the direct form. One pool
+// per device for all spaces. It keeps at most kContactMaxBytes that no call uses
+// (mapping fresh memory costs milliseconds per GB) and returns those to the
+// device when the last space on the device goes, or when an allocation of
+// the library fails.
+struct ScratchPool {
+    std::mutex mutex;
+    cudaMemPool_t pool[64] = {};
+    int spaces[64] = {};
+};
+ScratchPool &scratch()
+{
+    static ScratchPool *p = new ScratchPool;   // never destroyed: spaces may outlive static destructors
+    return *p;
+}
+
+cudaError_t pool_alloc(int device, void **ptr, size_t bytes, cudaStream_t st)
+{
+    ScratchPool &p = scratch();
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(p.mutex);
+        if (!p.pool[device]) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            cudaError_t e = cudaMemPoolCreate(&p.pool[device], &props);
+            uint64_t keep = mcpi::kContactMaxBytes;
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(p.pool[device], cudaMemPoolAttrReleaseThreshold, &keep);
+            if (e != cudaSuccess) return e;
+        }
+        pool = p.pool[device];
+    }
+    return cudaMallocFromPoolAsync(ptr, bytes, pool, st);
+}
+
+void pool_trim(int device)
+{
+    ScratchPool &p = scratch();
+    std::lock_guard<std::mutex> lock(p.mutex);
+    if (p.pool[device]) cudaMemPoolTrimTo(p.pool[device], 0);
+}
+
+// Counts the spaces of a device; the pool empties with the last one.
+void pool_space(int device, int step)
+{
+    ScratchPool &p = scratch();
+    std::lock_guard<std::mutex> lock(p.mutex);
+    p.spaces[device] += step;
+    if (p.spaces[device] == 0 && p.pool[device]) cudaMemPoolTrimTo(p.pool[device], 0);
+}
+
+// cudaMalloc, once more without the pool's unused memory when it fails for lack of it.
+template <class T>
+cudaError_t malloc_or_trim(int device, T **ptr, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    (void)cudaGetLastError();
+    pool_trim(device);
+    return cudaMalloc(ptr, bytes);
+}
+
+// The intermediate that the form of v passes between its halves: E (P x
+// NC(N-2,M)) of the two-kernel and fused forms, S ((2M-1) x NC(N-2,M)) of the
+// contact form where that stands in for them (elsewhere each call takes its S
+// from the pool below); the direct form needs none.
+int ensure_E(mcpi_space_s *sp, const PairOp &v)
 {
     if (sp->N < 2) return MCPI_OK;
-    if (mcpi::hpsi_form(sp->sp, op_view(sp, op)) == mcpi::kFormDirect) return MCPI_OK;
-    if (!sp->d_E) CK(cudaMalloc(&sp->d_E, sizeof(double2) * (size_t)sp->P * sp->nc2));
+    const int form = mcpi::hpsi_form(sp->sp, v);
+    if (form == mcpi::kFormContact) {
+        if (!sp->d_S && !mcpi::direct_covers(sp->sp)) CK(malloc_or_trim(sp->device, &sp->d_S, contact_bytes(sp)));
+        return MCPI_OK;
+    }
+    if (form == mcpi::kFormDirect) return MCPI_OK;
+    if (!sp->d_E) CK(malloc_or_trim(sp->device, &sp->d_E, sizeof(double2) * (size_t)sp->P * sp->nc2));
     return ensure_fused(sp);
+}
+
+// One H.psi on the space's stream.
+cudaError_t run_hpsi(mcpi_space_s *sp, const DevPairOp &op, PairOp v, const double2 *psi, double2 *out,
+                     int stages = 3, uint32_t row0 = 0, uint32_t row1 = 0xffffffffu, uint32_t m0 = 0,
+                     uint32_t m1 = 0xffffffffu)
+{
+    const cudaStream_t st = sp->stream;
+    double2 *scratch = sp->d_E;
+    void *S = nullptr;
+    if (mcpi::hpsi_form(sp->sp, v) == mcpi::kFormContact) {
+        scratch = sp->d_S;
+        if (mcpi::direct_covers(sp->sp)) {
+            if (contact_bytes(sp) > mcpi::kContactMaxBytes ||
+                pool_alloc(sp->device, &S, contact_bytes(sp), st) != cudaSuccess) {
+                (void)cudaGetLastError();
+                v.contact = nullptr;   // the direct form
+            }
+            scratch = (double2 *)S;
+        }
+    }
+    cudaError_t e = mcpi::launch_apply_h(sp->sp, sp->tables(), v, op.blocks(), psi, scratch, out, st, stages, row0,
+                                         row1, m0, m1);
+    if (S) {
+        const cudaError_t f = cudaFreeAsync(S, st);
+        if (e == cudaSuccess) e = f;
+    }
+    return e;
+}
+
+int reserve(mcpi_space_s *sp, void *&ptr, size_t &cap, size_t bytes)
+{
+    if (cap >= bytes && ptr) return MCPI_OK;
+    cudaFree(ptr);
+    ptr = nullptr;
+    cap = 0;
+    CK(malloc_or_trim(sp->device, &ptr, bytes ? bytes : 1));
+    cap = bytes;
+    return MCPI_OK;
 }
 
 void free_fused(mcpi_space_s *sp)
@@ -343,6 +486,15 @@ PairOp op_view(const mcpi_space_s *sp, const DevPairOp &op)
     PairOp v = op.view();
     if (sp->fused_on && sp->fz_ready) v.fused = sp->fz;
     v.direct = sp->direct_on;
+    if (sp->direct_on == 2 && !sp->fused_on && !op.contact.empty() &&
+        mcpi::contact_pays(sp->sp)) {
+        // under stream capture the direct form, which has no scratch, stays
+        // where there is one
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (!mcpi::direct_covers(sp->sp) ||
+            (cudaStreamIsCapturing(sp->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone))
+            v.contact = op.contact.data();
+    }
     return v;
 }
 
@@ -354,7 +506,7 @@ int ensure_gram(mcpi_space_s *sp)
     if (sp->gram_cap >= need) return MCPI_OK;
     cudaFree(sp->d_gram);
     sp->d_gram = nullptr;
-    CK(cudaMalloc(&sp->d_gram, sizeof(double2) * need));
+    CK(malloc_or_trim(sp->device, &sp->d_gram, sizeof(double2) * need));
     sp->gram_cap = need;
     return MCPI_OK;
 }
@@ -365,10 +517,10 @@ int apply_op(mcpi_space_s *sp, const DevPairOp &op, const void *d_C, void *d_out
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     CHECK_ARG(d_C != d_out, "input and output must not alias");
     DeviceGuard g(sp->device);
-    int rc = ensure_E(sp, op);
+    PairOp v = op_view(sp, op);
+    int rc = ensure_E(sp, v);
     if (rc) return rc;
-    CK(mcpi::launch_apply_h(sp->sp, sp->tables(), op_view(sp, op), op.blocks(), (const double2 *)d_C,
-                            sp->d_E, (double2 *)d_out, sp->stream));
+    CK(run_hpsi(sp, op, op_view(sp, op), (const double2 *)d_C, (double2 *)d_out));
     return MCPI_OK;
 }
 
@@ -428,9 +580,10 @@ int mcpi_space_create(int N, int M, int device, mcpi_space *out)
         return fail(MCPI_ERR_RANGE, "N=%d too large for the shared-memory binomial table", N);
     int ndev = 0;
     CK(cudaGetDeviceCount(&ndev));
-    CHECK_ARG(device >= 0 && device < ndev, "invalid device ordinal");
+    CHECK_ARG(device >= 0 && device < ndev && device < 64, "invalid device ordinal");
     DeviceGuard g(device);
     auto *s = new mcpi_space_s;
+    pool_space(device, 1);
     s->N = N;
     s->M = M;
     s->device = device;
@@ -526,6 +679,7 @@ int mcpi_space_destroy(mcpi_space sp)
     cudaFree(sp->d_W);
     cudaFree(sp->d_sq);
     cudaFree(sp->d_E);
+    cudaFree(sp->d_S);
     cudaFree(sp->d_gram);
     cudaFree(sp->d_dot);
     cudaFree(sp->d_status);
@@ -539,6 +693,7 @@ int mcpi_space_destroy(mcpi_space sp)
     free_fused(sp);
     cudaFree(sp->d_mr);
     if (sp->own) cudaStreamDestroy(sp->own);
+    pool_space(sp->device, -1);
     delete sp;
     return MCPI_OK;
 }
@@ -841,10 +996,20 @@ int mcpi_apply_h_host(mcpi_space sp, int count, const void *const *h_C, void *co
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     for (int k = 0; k < count; ++k) CHECK_ARG(h_C[k] && h_out[k], "mcpi_apply_h_host: null state pointer");
     DeviceGuard g(sp->device);
-    int rc = ensure_E(sp, sp->fwd);
+    PairOp fop = op_view(sp, sp->fwd);
+    int rc = ensure_E(sp, fop);
     if (rc) return rc;
     const size_t bytes = sizeof(double2) * (size_t)sp->nc;
-    if (!sp->host_pipe_ready) CK(make_host_pipe(sp, bytes));
+    if (!sp->host_pipe_ready) {
+        cudaError_t e = make_host_pipe(sp, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            (void)cudaGetLastError();
+            pool_trim(sp->device);
+            e = make_host_pipe(sp, bytes);
+        }
+        CK(e);
+    }
+    fop = op_view(sp, sp->fwd);
     // buffer pair b = k & 1: its input is free once H.psi of state k-2 has run,
     // its output once the copy out of state k-2 has finished
     for (int k = 0; k < count; ++k) {
@@ -854,8 +1019,7 @@ int mcpi_apply_h_host(mcpi_space sp, int count, const void *const *h_C, void *co
         CK(cudaEventRecord(sp->ev_in[b], sp->s_h2d));
         CK(cudaStreamWaitEvent(sp->stream, sp->ev_in[b], 0));
         if (k >= 2) CK(cudaStreamWaitEvent(sp->stream, sp->ev_out[b], 0));
-        CK(mcpi::launch_apply_h(sp->sp, sp->tables(), op_view(sp, sp->fwd), sp->fwd.blocks(), sp->d_hin[b], sp->d_E,
-                                sp->d_hout[b], sp->stream));
+        CK(run_hpsi(sp, sp->fwd, fop, sp->d_hin[b], sp->d_hout[b]));
         CK(cudaEventRecord(sp->ev_comp[b], sp->stream));
         CK(cudaStreamWaitEvent(sp->s_d2h, sp->ev_comp[b], 0));
         CK(cudaMemcpyAsync(h_out[k], sp->d_hout[b], bytes, cudaMemcpyDeviceToHost, sp->s_d2h));
@@ -871,21 +1035,36 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
     CHECK_ARG(sp && d_C && d_out && h_ms && reps >= 1, "mcpi_apply_h_profile: bad arguments");
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     DeviceGuard g(sp->device);
-    int rc = ensure_E(sp, sp->fwd);
+    PairOp fop = op_view(sp, sp->fwd);
+    int rc = ensure_E(sp, fop);
     if (rc) return rc;
+    fop = op_view(sp, sp->fwd);
     cudaEvent_t ev[3];
     for (auto &e : ev) CK(cudaEventCreate(&e));
     float tot[2] = {0.f, 0.f};
     cudaError_t e = cudaSuccess;
-    const PairOp fop = op_view(sp, sp->fwd);
-    const bool one = mcpi::hpsi_form(sp->sp, fop) != mcpi::kFormTwo;
+    // the contact form's two halves run apart here, on one S
+    double2 *scratch = sp->d_E;
+    void *S = nullptr;
+    if (mcpi::hpsi_form(sp->sp, fop) == mcpi::kFormContact) {
+        scratch = sp->d_S;
+        if (mcpi::direct_covers(sp->sp)) {
+            if (contact_bytes(sp) > mcpi::kContactMaxBytes ||
+                pool_alloc(sp->device, &S, contact_bytes(sp), sp->stream) != cudaSuccess) {
+                (void)cudaGetLastError();
+                fop.contact = nullptr;
+            }
+            scratch = (double2 *)S;
+        }
+    }
+    const int form = mcpi::hpsi_form(sp->sp, fop);
+    const bool one = form == mcpi::kFormDirect || form == mcpi::kFormFused;
     if (one) {
         // direct or fused form: one kernel, reported as h_ms[0]
         for (int r = 0; r < reps && e == cudaSuccess; ++r) {
             e = cudaEventRecord(ev[0], sp->stream);
             if (e == cudaSuccess)
-                e = mcpi::launch_apply_h(sp->sp, sp->tables(), fop, sp->fwd.blocks(), (const double2 *)d_C,
-                                         sp->d_E, (double2 *)d_out, sp->stream, 3);
+                e = run_hpsi(sp, sp->fwd, fop, (const double2 *)d_C, (double2 *)d_out);
             if (e == cudaSuccess) e = cudaEventRecord(ev[1], sp->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
             float a = 0.f;
@@ -896,12 +1075,12 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
     for (int r = 0; r < reps && e == cudaSuccess && !one; ++r) {
         e = cudaEventRecord(ev[0], sp->stream);
         if (e == cudaSuccess)
-            e = mcpi::launch_apply_h(sp->sp, sp->tables(), sp->fwd.view(), sp->fwd.blocks(),
-                                     (const double2 *)d_C, sp->d_E, (double2 *)d_out, sp->stream, 1);
+            e = mcpi::launch_apply_h(sp->sp, sp->tables(), fop, sp->fwd.blocks(), (const double2 *)d_C, scratch,
+                                     (double2 *)d_out, sp->stream, 1);
         if (e == cudaSuccess) e = cudaEventRecord(ev[1], sp->stream);
         if (e == cudaSuccess)
-            e = mcpi::launch_apply_h(sp->sp, sp->tables(), sp->fwd.view(), sp->fwd.blocks(),
-                                     (const double2 *)d_C, sp->d_E, (double2 *)d_out, sp->stream, 2);
+            e = mcpi::launch_apply_h(sp->sp, sp->tables(), fop, sp->fwd.blocks(), (const double2 *)d_C, scratch,
+                                     (double2 *)d_out, sp->stream, 2);
         if (e == cudaSuccess) e = cudaEventRecord(ev[2], sp->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(ev[2]);
         float a = 0.f, b = 0.f;
@@ -911,6 +1090,7 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
         tot[1] += b;
     }
     for (auto &x : ev) cudaEventDestroy(x);
+    if (S) cudaFreeAsync(S, sp->stream);
     if (e != cudaSuccess) return fail(MCPI_ERR_CUDA, "mcpi_apply_h_profile: %s", cudaGetErrorString(e));
     h_ms[0] = tot[0] / reps;
     h_ms[1] = tot[1] / reps;
@@ -927,14 +1107,20 @@ int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1
     if (sp->N < 2 || sp->create_form != 0)
         return fail(MCPI_ERR_ARG, "row ranges need N >= 2 and the default pair-creation form");
     DeviceGuard g(sp->device);
-    int rc = ensure_E(sp, sp->fwd);
+    // a part of the rows takes the direct form where there is one: its work is
+    // exactly the rows', while the contact form's first half covers every
+    // configuration that they read
+    const bool part = row0 != 0 || row1 != sp->nc;
+    PairOp fop = op_view(sp, sp->fwd);
+    if (part && mcpi::direct_covers(sp->sp)) fop.contact = nullptr;
+    int rc = ensure_E(sp, fop);
     if (rc) return rc;
+    if (sp->fz_ready) fop = op_view(sp, sp->fwd);
     // kernel 1 only over the E columns these rows read (momentum-block form):
     // a rank of a sharded solve does not recompute the whole intermediate.
     // The range is found once per row block (one pass over its rows).
     uint32_t m0 = 0, m1 = 0xffffffffu;
-    const PairOp fop = op_view(sp, sp->fwd);
-    if (sp->fwd.hblk && sp->M >= 2 && mcpi::hpsi_form(sp->sp, fop) != mcpi::kFormDirect) {
+    if (part && sp->fwd.hblk && sp->M >= 2 && mcpi::hpsi_form(sp->sp, fop) != mcpi::kFormDirect) {
         if (sp->mr_r0 != row0 || sp->mr_r1 != row1) {
             if (!sp->d_mr) CK(cudaMalloc(&sp->d_mr, 2 * sizeof(uint32_t)));
             uint32_t h[2];
@@ -950,8 +1136,7 @@ int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1
         m0 = sp->mr_lo;
         m1 = sp->mr_hi + 1;
     }
-    CK(mcpi::launch_apply_h(sp->sp, sp->tables(), fop, sp->fwd.blocks(), (const double2 *)d_C,
-                            sp->d_E, (double2 *)d_out, sp->stream, 3, (uint32_t)row0, (uint32_t)row1, m0, m1));
+    CK(run_hpsi(sp, sp->fwd, fop, (const double2 *)d_C, (double2 *)d_out, 3, (uint32_t)row0, (uint32_t)row1, m0, m1));
     return MCPI_OK;
 }
 
@@ -1079,15 +1264,16 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
     CHECK_ARG(sp && d_lvec && lm >= 1, "mcpi_lanczos: bad arguments");
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     DeviceGuard g(sp->device);
-    int rc = ensure_E(sp, sp->fwd);
+    PairOp op = op_view(sp, sp->fwd);
+    int rc = ensure_E(sp, op);
     if (rc) return rc;
     const int64_t nc = sp->nc;
     const size_t npart = mcpi::lanczos_partial_elems(nc, lm);
     // state block: alpha(lm) coef(lm) partial(npart) | beta(lm) maxbeta | done iters
     const size_t bytes = sizeof(double2) * (2 * (size_t)lm + npart) + sizeof(double) * (lm + 1) + 2 * sizeof(int);
-    rc = reserve(sp->d_lzblk, sp->lzblk_cap, bytes);
+    rc = reserve(sp, sp->d_lzblk, sp->lzblk_cap, bytes);
     if (rc) return rc;
-    rc = reserve(sp->d_lzr, sp->lzr_cap, sizeof(double2) * nc);
+    rc = reserve(sp, sp->d_lzr, sp->lzr_cap, sizeof(double2) * nc);
     if (rc) return rc;
     char *blk = (char *)sp->d_lzblk;
     double2 *r = (double2 *)sp->d_lzr;
@@ -1103,18 +1289,16 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
     s.nparts = mcpi::lanczos_parts(nc);
     const int init[2] = {0, lm};
     double2 *V = (double2 *)d_lvec;
-    const PairOp op = op_view(sp, sp->fwd);
-    const mcpi::BlockOp bo = sp->fwd.blocks();
-    const SpaceTables tb = sp->tables();
+    op = op_view(sp, sp->fwd);
     e = cudaMemsetAsync(blk, 0, bytes, sp->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s.done, init, sizeof init, cudaMemcpyHostToDevice, sp->stream);
-    if (e == cudaSuccess) e = mcpi::launch_apply_h(sp->sp, tb, op, bo, V, sp->d_E, r, sp->stream);
+    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, V, r);
     if (e == cudaSuccess) e = mcpi::launch_lanczos_start(V, r, r, nc, s, sp->stream);
     for (int i = 0; i < lm - 1 && e == cudaSuccess; ++i) {
         double2 *vi = V + (size_t)i * nc, *vn = V + (size_t)(i + 1) * nc;
         e = mcpi::launch_lanczos_beta(i, lm, 1e-15, s, sp->stream);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, sp->stream);
-        if (e == cudaSuccess) e = mcpi::launch_apply_h(sp->sp, tb, op, bo, vn, sp->d_E, r, sp->stream);
+        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, vn, r);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_alpha(vi, vn, r, nc, i, s, sp->stream);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_reorth(V, i + 2, r, nc, i, s, sp->stream);
     }
@@ -1148,7 +1332,7 @@ int mcpi_ground(mcpi_space sp, void *d_C, int niter, double *E0, int *iters)
     CHECK_ARG(sp && d_C && E0 && niter >= 1, "mcpi_ground: bad arguments");
     DeviceGuard g(sp->device);
     const int64_t nc = sp->nc;
-    int rc0 = reserve(sp->d_basis, sp->basis_cap, sizeof(double2) * nc * (size_t)niter);
+    int rc0 = reserve(sp, sp->d_basis, sp->basis_cap, sizeof(double2) * nc * (size_t)niter);
     if (rc0) return rc0;
     double2 *V = (double2 *)sp->d_basis;
     cudaError_t e = cudaMemcpyAsync(V, d_C, sizeof(double2) * nc, cudaMemcpyDeviceToDevice, sp->stream);
@@ -1195,7 +1379,8 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     CHECK_ARG(sp && d_C && E0 && niter >= 1 && niter <= 1 << 20, "mcpi_ground_lowmem: bad arguments");
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     DeviceGuard g(sp->device);
-    int rc = ensure_E(sp, sp->fwd);
+    PairOp op = op_view(sp, sp->fwd);
+    int rc = ensure_E(sp, op);
     if (rc) return rc;
     const int64_t nc = sp->nc;
     const int lm = niter;
@@ -1205,8 +1390,8 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
                           2 * sizeof(int);
     char *blk = nullptr;
     double2 *vec = nullptr;   // v[0], v[1], r, acc
-    CK(cudaMalloc(&blk, sbytes));
-    cudaError_t e = cudaMalloc(&vec, sizeof(double2) * nc * 4);
+    CK(malloc_or_trim(sp->device, &blk, sbytes));
+    cudaError_t e = malloc_or_trim(sp->device, &vec, sizeof(double2) * nc * 4);
     if (e != cudaSuccess) {
         cudaFree(blk);
         return fail(MCPI_ERR_NOMEM, "mcpi_ground_lowmem: %s", cudaGetErrorString(e));
@@ -1222,22 +1407,20 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     s.iters = s.done + 1;
     s.nparts = mcpi::lanczos_parts(nc);
     double2 *v[2] = {vec, vec + nc}, *r = vec + 2 * nc, *acc = vec + 3 * nc;
-    const PairOp op = op_view(sp, sp->fwd);
-    const mcpi::BlockOp bo = sp->fwd.blocks();
-    const SpaceTables tb = sp->tables();
+    op = op_view(sp, sp->fwd);
     const int init[2] = {0, lm};
     cudaStream_t st = sp->stream;
     // pass 1: tridiagonal only
     e = cudaMemsetAsync(blk, 0, sbytes, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s.done, init, sizeof init, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(v[0], d_C, sizeof(double2) * nc, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = mcpi::launch_apply_h(sp->sp, tb, op, bo, v[0], sp->d_E, r, st);
+    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, v[0], r);
     if (e == cudaSuccess) e = mcpi::launch_lanczos_start(v[0], r, r, nc, s, st);
     for (int i = 0; i < lm - 1 && e == cudaSuccess; ++i) {
         double2 *vi = v[i & 1], *vn = v[(i + 1) & 1];
         e = mcpi::launch_lanczos_beta(i, lm, 1e-15, s, st);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, st);
-        if (e == cudaSuccess) e = mcpi::launch_apply_h(sp->sp, tb, op, bo, vn, sp->d_E, r, st);
+        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, vn, r);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_alpha(vi, vn, r, nc, i, s, st);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_no_reorth(vn, r, nc, i, s, st);
     }
@@ -1271,13 +1454,13 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     if (e == cudaSuccess) e = cudaMemcpyAsync(dz, zc.data(), sizeof(double) * lm, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s.done, init, sizeof init, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(v[0], d_C, sizeof(double2) * nc, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = mcpi::launch_apply_h(sp->sp, tb, op, bo, v[0], sp->d_E, r, st);
+    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, v[0], r);
     if (e == cudaSuccess) e = mcpi::launch_lanczos_no_reorth(v[0], r, nc, -1, s, st);
     if (e == cudaSuccess) e = mcpi::launch_axpy_real(acc, v[0], nc, dz, 1, st);
     for (int i = 0; i < n - 1 && e == cudaSuccess; ++i) {
         double2 *vi = v[i & 1], *vn = v[(i + 1) & 1];
         e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, st);
-        if (e == cudaSuccess) e = mcpi::launch_apply_h(sp->sp, tb, op, bo, vn, sp->d_E, r, st);
+        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, vn, r);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_axpy(vi, r, nc, i, s, st);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_no_reorth(vn, r, nc, i, s, st);
         if (e == cudaSuccess) e = mcpi::launch_axpy_real(acc, vn, nc, dz + i + 1, 0, st);

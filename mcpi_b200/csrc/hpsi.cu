@@ -1209,6 +1209,184 @@ cudaError_t direct_apply_m(const Space &sp, const SpaceTables &tb, const PairOp 
     return launch_direct<M, false>(sp, tb, hp, op.hdiag, psi, out, st, row0, row1);
 }
 
+// ---------------------------------------------------------------------------
+// H.psi, contact form. A contact interaction couples every pair of total K to
+// every other with one strength, so each momentum block is an outer product
+// Ht[a][b] = u_a w_b (real; found on the host from the values themselves,
+// capi.cpp pack_contact) and the pair-space product collapses to one sum per
+// total momentum instead of one per creation pair:
+//     S_K(m) = sum_{b in block K} w_b c_b(m) psi[m + b],
+//     (H2 psi)(v) = sum_{a in v} u_a c_a(v) S_{K(a)}(v - a).
+// ---------------------------------------------------------------------------
+template <int M>
+struct ContactVals {
+    static constexpr int P = M * (M + 1) / 2;
+    double u[P], w[P];   // in pair_index order
+};
+
+template <int M>
+__global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb,
+                                                     const __grid_constant__ ContactVals<M> cv,
+                                                     const double2 *__restrict__ psi, double2 *__restrict__ S,
+                                                     uint32_t m0, uint32_t m1)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *sq = reinterpret_cast<double *>(smem_raw);            // wstride
+    uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);  // (M-1) x wstride
+    load_tables(sp, tb, W, sq);
+    __syncthreads();
+    const uint32_t m = m0 + blockIdx.x * kT2 + threadIdx.x;
+    if (m >= m1) return;
+    const int ws = sp.wstride;
+    int u[M], Q[M];
+    occupations<M>(tb.occ2, tb.occ_bits, m, sp.N - 2, sp.nc2, W, ws, u, Q);
+    double fa[M];
+    uint32_t Xa[M], Ya[M];   // index(m + e_q + e_l) = Xa[q] - Ya[l]  (q <= l)
+    {
+        uint32_t B0[M], B1[M], B2[M];
+        prefix_table<M>(Q, 0, W, ws, B0);
+        prefix_table<M>(Q, 1, W, ws, B1);
+        prefix_table<M>(Q, 2, W, ws, B2);
+        const uint32_t base = sp.nc - 1u - B2[M - 1];
+#pragma unroll
+        for (int o = 0; o < M; ++o) {
+            fa[o] = sq[u[o] + 1];
+            Xa[o] = base - (B0[o] - B1[o]);
+            Ya[o] = B1[o] - B2[o];
+        }
+    }
+    const size_t stride = sp.nc2;
+    constexpr int NB = M / 2 + 1;   // widest block
+#pragma unroll
+    for (int K = 0; K <= 2 * M - 2; ++K) {
+        const int qlo = K - (M - 1) > 0 ? K - (M - 1) : 0, qhi = K / 2, n = qhi - qlo + 1;
+        double2 x[NB];
+#pragma unroll
+        for (int c = 0; c < NB; ++c)
+            if (c < n) x[c] = __ldg(psi + (Xa[qlo + c] - Ya[K - qlo - c]));
+        double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int c = 0; c < NB; ++c)
+            if (c < n) {
+                const int q = qlo + c, l = K - q;
+                const double f = cv.w[pair_index(q, l, M)] * (fa[q] * ((q == l) ? sq[u[q] + 2] : fa[l]));
+                s.x = fma(f, x[c].x, s.x);
+                s.y = fma(f, x[c].y, s.y);
+            }
+        S[K * stride + m] = s;
+    }
+}
+
+template <int M>
+__global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables tb,
+                                                        const __grid_constant__ ContactVals<M> cv,
+                                                        const double2 *__restrict__ hdiag,
+                                                        const double2 *__restrict__ psi,
+                                                        const double2 *__restrict__ S, double2 *__restrict__ out,
+                                                        uint32_t row0, uint32_t row1)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *r1 = reinterpret_cast<double *>(smem_raw);             // M x kTC
+    uint32_t *Xr = reinterpret_cast<uint32_t *>(r1 + M * kTC);     // M x kTC
+    uint32_t *Yr = Xr + M * kTC;                                   // M x kTC
+    unsigned char *vb = reinterpret_cast<unsigned char *>(Yr + M * kTC);   // M x kTC
+    double2 *hd = reinterpret_cast<double2 *>(vb + ((M * kTC + 15) & ~15)); // M
+    double *sq = reinterpret_cast<double *>(hd + M);               // wstride
+    uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);   // (M-1) x wstride
+    load_tables(sp, tb, W, sq);
+    if (threadIdx.x < M) hd[threadIdx.x] = hdiag[threadIdx.x];
+    __syncthreads();
+    // from the top rows down: their S entries were written last, some are still in L2
+    const uint32_t i = row0 + (gridDim.x - 1 - blockIdx.x) * kTC + threadIdx.x;
+    if (i >= row1) return;
+    const int t = threadIdx.x, ws = sp.wstride;
+    double2 acc;
+    {
+        int v[M], P[M];
+        occupations<M>(tb.occ, tb.occ_bits, i, sp.N, sp.nc, W, ws, v, P);
+        double2 h1 = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < M; ++k) {
+            h1.x += hd[k].x * v[k];
+            h1.y += hd[k].y * v[k];
+        }
+        acc = cmul(h1, psi[i]);
+        uint32_t A0[M], Am1[M], Am2[M];
+        prefix_table<M>(P, 0, W, ws, A0);
+        prefix_table<M>(P, -1, W, ws, Am1);
+        prefix_table<M>(P, -2, W, ws, Am2);
+        const uint32_t base = sp.nc2 - 1u - Am2[M - 1];
+#pragma unroll
+        for (int o = 0; o < M; ++o) {
+            Xr[o * kTC + t] = base - (A0[o] - Am1[o]);
+            Yr[o * kTC + t] = Am1[o] - Am2[o];
+            r1[o * kTC + t] = sq[v[o]];
+            vb[o * kTC + t] = (unsigned char)(v[o] >= 1 ? v[o] - 1 : 0);
+        }
+    }
+    const size_t stride = sp.nc2;
+    constexpr int NPR = M * (M + 1) / 2;
+#pragma unroll
+    for (int p0 = 0; p0 < NPR; p0 += kCreateBatch) {
+        double cc[kCreateBatch];
+        double2 ee[kCreateBatch];
+#pragma unroll
+        for (int j = 0; j < kCreateBatch; ++j) {
+            const int p = p0 + j;
+            if (p < NPR) {
+                int k = 0, rem = p;   // (k, s) of pair p, resolved at compile time
+#pragma unroll
+                for (int kk = 0; kk < M; ++kk)
+                    if (rem >= M - kk && k == kk) {
+                        rem -= M - kk;
+                        k = kk + 1;
+                    }
+                const int s = k + rem;
+                const double c = r1[k * kTC + t] * ((s == k) ? sq[vb[k * kTC + t]] : r1[s * kTC + t]);
+                const uint32_t mm = Xr[k * kTC + t] - Yr[s * kTC + t];
+                cc[j] = c * cv.u[p];
+                ee[j] = c == 0.0 ? make_double2(0.0, 0.0) : __ldg(S + (size_t)(k + s) * stride + mm);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kCreateBatch; ++j)
+            if (p0 + j < NPR) {
+                acc.x = fma(cc[j], ee[j].x, acc.x);
+                acc.y = fma(cc[j], ee[j].y, acc.y);
+            }
+    }
+    out[i - row0] = acc;
+}
+
+template <int M>
+cudaError_t contact_apply_m(const Space &sp, const SpaceTables &tb, const PairOp &op, const double2 *psi, double2 *S,
+                            double2 *out, int stages, cudaStream_t st, uint32_t row0, uint32_t row1, uint32_t m0,
+                            uint32_t m1)
+{
+    constexpr int P = M * (M + 1) / 2;
+    ContactVals<M> cv;
+    for (int x = 0; x < P; ++x) {
+        cv.u[x] = op.contact[x];
+        cv.w[x] = op.contact[P + x];
+    }
+    const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
+    if (m1 > sp.nc2) m1 = sp.nc2;
+    if ((stages & 1) && m1 > m0)
+        k_contact_sum<M><<<(m1 - m0 + kT2 - 1) / kT2, kT2, tab, st>>>(sp, tb, cv, psi, S, m0, m1);
+    if ((stages & 2) && row1 > row0) {
+        const size_t sm = (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + ((M * kTC + 15) & ~15) +
+                          sizeof(double2) * M + tab;
+        if (sm > 48 * 1024) {
+            const cudaError_t e = cudaFuncSetAttribute(k_contact_create<M>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            if (e != cudaSuccess) return e;
+        }
+        k_contact_create<M><<<(row1 - row0 + kTC - 1) / kTC, kTC, sm, st>>>(sp, tb, cv, op.hdiag, psi, S, out, row0,
+                                                                          row1);
+    }
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 // Number of momentum-block values for M orbitals, at run time.
@@ -1222,9 +1400,20 @@ static int mom_count(int M)
     return s;
 }
 
+bool contact_pays(const Space &sp)
+{
+    if (!direct_covers(sp)) return true;   // stands in for the two pair kernels
+    // against the direct form, measured in us (contact / direct) on rotating
+    // states: M=11 N=10 33 / 35, N=12 77 / 97, N=16 582 / 750; M=10 N=11 28 / 25,
+    // N=12 37 / 37, N=13 58 / 74, N=16 205 / 226, N=18 475 / 512, N=20 1154 / 1117
+    // (S then no longer has a useful share in L2); M=9 N=16 75 / 68, N=20 294 / 274
+    return sp.M == 11 ? sp.nc >= 180000 : sp.M == 10 && sp.nc >= 290000 && sp.nc <= 6000000;
+}
+
 int hpsi_form(const Space &sp, const PairOp &op)
 {
     if (sp.N < 2 || sp.M < 2 || !op.hblk_host || op.nhblk != mom_count(sp.M)) return kFormTwo;
+    if (op.contact && op.create_form == 0) return kFormContact;
     // N < 64 bounds the square-root product table, (N + 3)^2 doubles of shared memory
     if (op.direct && sp.N < 64 && op.create_form == 0 && (op.direct != 2 || sp.M <= kDirectAutoMaxM))
         return kFormDirect;
@@ -1625,8 +1814,10 @@ cudaError_t apply_h_m(const Space &sp, const SpaceTables &tb, const PairOp &op, 
     constexpr int P = M * (M + 1) / 2;
     const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
     if constexpr (M >= 2) {
+        const int form = hpsi_form(sp, op);
+        if (form == kFormContact)
+            return contact_apply_m<M>(sp, tb, op, psi, E, out, stages, st, row0, row1, m0, m1);
         if (stages == 3) {
-            const int form = hpsi_form(sp, op);
             if (form == kFormDirect) return direct_apply_m<M>(sp, tb, op, psi, out, st, row0, row1);
             if (form == kFormFused && row0 == 0 && row1 == sp.nc)
                 return fused_apply_m<M>(sp, tb, op, psi, E, out, st);

@@ -62,12 +62,23 @@ struct PairOp {
     // direct form: momentum-block integrals applied row by row with no
     // intermediate (0 off, 1 on, 2 on for M <= kDirectAutoMaxM)
     int direct;
+    // contact form: every momentum block is an outer product u_a w_b of real
+    // factors (host array u[P] | w[P] in pair_index order, null otherwise)
+    const double *contact;
 };
 
 // The form a whole-vector H.psi (both stages, all rows) takes with op.
-enum { kFormTwo = 0, kFormFused = 1, kFormDirect = 2 };
+enum { kFormTwo = 0, kFormFused = 1, kFormDirect = 2, kFormContact = 3 };
 constexpr int kDirectAutoMaxM = 11;
 int hpsi_form(const Space &sp, const PairOp &op);
+// The spaces whose momentum-block integrals take the direct form by default.
+// N < 64 bounds its square-root product table, (N + 3)^2 doubles of shared memory.
+inline bool direct_covers(const Space &sp) { return sp.M <= kDirectAutoMaxM && sp.N < 64; }
+// Whether the contact form is faster than the form it would stand in for, and
+// the most device memory that its intermediate may take where the direct form
+// can run instead (what the pool of capi.cpp keeps between calls).
+bool contact_pays(const Space &sp);
+constexpr size_t kContactMaxBytes = (size_t)2 << 30;
 constexpr int kGemmMaxP = 78;   // M <= 12: Ht (zero-padded to a multiple of 8 rows) fits shared memory
 
 // Block-sparse form of the same pair matrix: when Ht decomposes into blocks

@@ -23,6 +23,7 @@ struct DevPairOp {
     double2 *hblk = nullptr;   // momentum-block form (nullptr when Ht couples different q+l)
     int nhblk = 0;
     std::vector<double2> hblk_h;   // host copy of hblk
+    std::vector<double> contact;   // outer-product factors u[P] | w[P] of the blocks (empty: not of that form)
     int create_form = 0;
     int *status = nullptr;     // the space's device status word (not owned)
     double2 *hdense = nullptr; // dense form (nullptr unless Ht is general and P <= kGemmMaxP)
@@ -31,7 +32,7 @@ struct DevPairOp {
     PairOp view() const
     {
         return PairOp{rowptr, col, val, hdiag, hfull, nnz, hblk, nhblk, create_form, status, hdense,
-                      wait_cycles, test_stall, hblk_h.empty() ? nullptr : hblk_h.data(), FusedPlan{}, 0};
+                      wait_cycles, test_stall, hblk_h.empty() ? nullptr : hblk_h.data(), FusedPlan{}, 0, nullptr};
     }
     BlockOp blocks() const { return BlockOp{prog, prog_bytes}; }
 };
@@ -57,6 +58,7 @@ struct mcpi_space_s {
     bool has_op = false;
     mcpi::DevPairOp fwd, adj;
     double2 *d_E = nullptr;          // P * nc2 scratch of H.psi
+    double2 *d_S = nullptr;          // (2M-1) * nc2 scratch of the contact form (spaces the direct form does not cover)
     double2 *d_gram = nullptr;       // density partials
     size_t gram_cap = 0;
     double2 *d_dot = nullptr;        // 1 result + partials
