@@ -21,6 +21,7 @@
 
 namespace mcpi {
 int tridiag_eig(int n, double *d, const double *e, double *z);
+int tridiag_lowest(int n, double *d, const double *e, double *E, double *z);
 }
 
 using mcpi::DevPairOp;
@@ -495,6 +496,19 @@ PairOp op_view(const mcpi_space_s *sp, const DevPairOp &op)
             (cudaStreamIsCapturing(sp->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone))
             v.contact = op.contact.data();
     }
+    return v;
+}
+
+// The view that a Lanczos recurrence takes. With an odd number of plane waves
+// the momenta are symmetric and the spectrum is doubly degenerate; once the
+// top pair has converged (about step 64 at N=5, M=11) the recurrence amplifies
+// rounding to order one, and with it the sign of the Ritz vector (measured
+// between any two forms of H.psi; E0 agrees to 1e-15). The form there stays
+// what it has been, so that a solve's vector does not change its sign.
+PairOp lanczos_view(const mcpi_space_s *sp)
+{
+    PairOp v = op_view(sp, sp->fwd);
+    if (sp->M & 1) v.contact = nullptr;
     return v;
 }
 
@@ -1264,7 +1278,7 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
     CHECK_ARG(sp && d_lvec && lm >= 1, "mcpi_lanczos: bad arguments");
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     DeviceGuard g(sp->device);
-    PairOp op = op_view(sp, sp->fwd);
+    PairOp op = lanczos_view(sp);
     int rc = ensure_E(sp, op);
     if (rc) return rc;
     const int64_t nc = sp->nc;
@@ -1289,7 +1303,7 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
     s.nparts = mcpi::lanczos_parts(nc);
     const int init[2] = {0, lm};
     double2 *V = (double2 *)d_lvec;
-    op = op_view(sp, sp->fwd);
+    op = lanczos_view(sp);
     e = cudaMemsetAsync(blk, 0, bytes, sp->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s.done, init, sizeof init, cudaMemcpyHostToDevice, sp->stream);
     if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, V, r);
@@ -1343,20 +1357,12 @@ int mcpi_ground(mcpi_space sp, void *d_C, int niter, double *E0, int *iters)
     if (rc) return rc;
     // groundStateLieb.c:419-449; a breakdown at the first step keeps alpha_0
     const int n = it > 0 ? it : 1;
-    std::vector<double> d(n), ee(n > 1 ? n - 1 : 1), z((size_t)n * n);
+    std::vector<double> d(n), ee(n > 1 ? n - 1 : 1), zc(n);
     for (int k = 0; k < n; ++k) d[k] = diag[2 * k];
     for (int k = 0; k + 1 < n; ++k) ee[k] = off[k];
-    if (mcpi::tridiag_eig(n, d.data(), ee.data(), z.data()) != 0)
+    double Emin = 0.0;
+    if (mcpi::tridiag_lowest(n, d.data(), ee.data(), &Emin, zc.data()) != 0)
         return fail(MCPI_ERR_NUMERIC, "tridiagonal QL did not converge");
-    double sentinel = 1e10;
-    int jmin = 0;
-    for (int k = 0; k < n; ++k)
-        if (sentinel > d[k]) {
-            sentinel = d[k];
-            jmin = k;
-        }
-    std::vector<double> zc(n);
-    for (int k = 0; k < n; ++k) zc[k] = z[(size_t)k * n + jmin];
     double *dz = nullptr;
     e = cudaMalloc(&dz, sizeof(double) * n);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dz, zc.data(), sizeof(double) * n, cudaMemcpyHostToDevice, sp->stream);
@@ -1364,7 +1370,7 @@ int mcpi_ground(mcpi_space sp, void *d_C, int niter, double *E0, int *iters)
     if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);
     cudaFree(dz);
     if (e != cudaSuccess) return fail(MCPI_ERR_CUDA, "mcpi_ground: %s", cudaGetErrorString(e));
-    *E0 = d[jmin];
+    *E0 = Emin;
     if (iters) *iters = it;
     return MCPI_OK;
 }
@@ -1379,7 +1385,7 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     CHECK_ARG(sp && d_C && E0 && niter >= 1 && niter <= 1 << 20, "mcpi_ground_lowmem: bad arguments");
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     DeviceGuard g(sp->device);
-    PairOp op = op_view(sp, sp->fwd);
+    PairOp op = lanczos_view(sp);
     int rc = ensure_E(sp, op);
     if (rc) return rc;
     const int64_t nc = sp->nc;
@@ -1407,7 +1413,7 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     s.iters = s.done + 1;
     s.nparts = mcpi::lanczos_parts(nc);
     double2 *v[2] = {vec, vec + nc}, *r = vec + 2 * nc, *acc = vec + 3 * nc;
-    op = op_view(sp, sp->fwd);
+    op = lanczos_view(sp);
     const int init[2] = {0, lm};
     cudaStream_t st = sp->stream;
     // pass 1: tridiagonal only
@@ -1432,23 +1438,16 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     if (e == cudaSuccess) e = cudaMemcpyAsync(&it, s.iters, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     const int n = it > 0 ? it : 1;
-    std::vector<double> d(n), ee(n > 1 ? n - 1 : 1), z((size_t)n * n), zc(lm, 0.0);
-    int jmin = 0;
+    std::vector<double> d(n), ee(n > 1 ? n - 1 : 1), zc(lm, 0.0);
+    double Emin = 0.0;
     if (e == cudaSuccess) {
         for (int k = 0; k < n; ++k) d[k] = alpha[k].x;
         for (int k = 0; k + 1 < n; ++k) ee[k] = beta[k];
-        if (mcpi::tridiag_eig(n, d.data(), ee.data(), z.data()) != 0) {
+        if (mcpi::tridiag_lowest(n, d.data(), ee.data(), &Emin, zc.data()) != 0) {
             cudaFree(blk);
             cudaFree(vec);
             return fail(MCPI_ERR_NUMERIC, "tridiagonal QL did not converge");
         }
-        double sentinel = 1e10;
-        for (int k = 0; k < n; ++k)
-            if (sentinel > d[k]) {
-                sentinel = d[k];
-                jmin = k;
-            }
-        for (int k = 0; k < n; ++k) zc[k] = z[(size_t)k * n + jmin];
     }
     // pass 2: regenerate v_0 .. v_{n-1} and accumulate sum_k z_k v_k
     if (e == cudaSuccess) e = cudaMemcpyAsync(dz, zc.data(), sizeof(double) * lm, cudaMemcpyHostToDevice, st);
@@ -1470,7 +1469,7 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     cudaFree(blk);
     cudaFree(vec);
     if (e != cudaSuccess) return fail(MCPI_ERR_CUDA, "mcpi_ground_lowmem: %s", cudaGetErrorString(e));
-    *E0 = d[jmin];
+    *E0 = Emin;
     if (iters) *iters = it;
     return check_status(sp);
 }
