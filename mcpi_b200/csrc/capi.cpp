@@ -267,6 +267,9 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
         op.hblk_h.resize(mom.size());
         std::memcpy(op.hblk_h.data(), mom.data(), sizeof(double2) * mom.size());
         op.contact = pack_contact(Ht, P, M);
+        op.real = true;
+        for (const cplx &h : mom) op.real = op.real && h.imag() == 0.0;
+        for (int k = 0; k < M; ++k) op.real = op.real && hdiag[k].imag() == 0.0;
     }
     const std::vector<int> prog = pack_blocks(Ht, P, M);
     if (!prog.empty() && !sp->dense_only) {
@@ -384,7 +387,7 @@ int ensure_E(mcpi_space_s *sp, const PairOp &v)
 }
 
 // One H.psi on the space's stream.
-cudaError_t run_hpsi(mcpi_space_s *sp, const DevPairOp &op, PairOp v, const double2 *psi, double2 *out,
+cudaError_t run_hpsi(mcpi_space_s *sp, const DevPairOp &op, PairOp &v, const double2 *psi, double2 *out,
                      int stages = 3, uint32_t row0 = 0, uint32_t row1 = 0xffffffffu, uint32_t m0 = 0,
                      uint32_t m1 = 0xffffffffu)
 {
@@ -534,7 +537,8 @@ int apply_op(mcpi_space_s *sp, const DevPairOp &op, const void *d_C, void *d_out
     PairOp v = op_view(sp, op);
     int rc = ensure_E(sp, v);
     if (rc) return rc;
-    CK(run_hpsi(sp, op, op_view(sp, op), (const double2 *)d_C, (double2 *)d_out));
+    if (sp->fz_ready) v = op_view(sp, op);   // the schedule that ensure_E may have built
+    CK(run_hpsi(sp, op, v, (const double2 *)d_C, (double2 *)d_out));
     return MCPI_OK;
 }
 
@@ -703,6 +707,7 @@ int mcpi_space_destroy(mcpi_space sp)
     cudaFree(sp->d_basis);
     cudaFree(sp->d_lzblk);
     cudaFree(sp->d_lzr);
+    cudaFree(sp->d_small);
     free_host_pipe(sp);
     free_fused(sp);
     cudaFree(sp->d_mr);
@@ -1273,6 +1278,14 @@ int mcpi_dot(mcpi_space sp, const void *d_a, const void *d_b, double *h_result2)
 
 // ---- Lanczos -------------------------------------------------------------------------
 
+// Whether a solve takes the one-launch form: real momentum-block operators with
+// no other form asked for, on a space and step count that it is made for.
+static bool small_lanczos(const mcpi_space_s *sp, int lm)
+{
+    return sp->direct_on == 2 && !sp->fused_on && sp->create_form == 0 && sp->fwd.real &&
+           mcpi::small_lanczos_fits(sp->sp, lm);
+}
+
 int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_offdiag, int *iters)
 {
     CHECK_ARG(sp && d_lvec && lm >= 1, "mcpi_lanczos: bad arguments");
@@ -1289,6 +1302,11 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
     if (rc) return rc;
     rc = reserve(sp, sp->d_lzr, sp->lzr_cap, sizeof(double2) * nc);
     if (rc) return rc;
+    const bool small = small_lanczos(sp, lm);
+    if (small) {
+        rc = reserve(sp, sp->d_small, sp->small_cap, mcpi::small_lanczos_bytes(sp->sp, lm));
+        if (rc) return rc;
+    }
     char *blk = (char *)sp->d_lzblk;
     double2 *r = (double2 *)sp->d_lzr;
     cudaError_t e = cudaSuccess;
@@ -1306,9 +1324,21 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
     op = lanczos_view(sp);
     e = cudaMemsetAsync(blk, 0, bytes, sp->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s.done, init, sizeof init, cudaMemcpyHostToDevice, sp->stream);
-    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, V, r);
-    if (e == cudaSuccess) e = mcpi::launch_lanczos_start(V, r, r, nc, s, sp->stream);
-    for (int i = 0; i < lm - 1 && e == cudaSuccess; ++i) {
+    bool one_launch = small && e == cudaSuccess;
+    if (one_launch) {
+        e = mcpi::launch_small_lanczos(sp->sp, sp->tables(), op, V, lm, 1e-15, r, s, sp->d_small, sp->device,
+                                       sp->stream);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            (void)cudaGetLastError();
+            e = cudaSuccess;
+            one_launch = false;
+        }
+    }
+    if (!one_launch) {
+        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, V, r);
+        if (e == cudaSuccess) e = mcpi::launch_lanczos_start(V, r, r, nc, s, sp->stream);
+    }
+    for (int i = 0; i < lm - 1 && e == cudaSuccess && !one_launch; ++i) {
         double2 *vi = V + (size_t)i * nc, *vn = V + (size_t)(i + 1) * nc;
         e = mcpi::launch_lanczos_beta(i, lm, 1e-15, s, sp->stream);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, sp->stream);

@@ -243,6 +243,19 @@ cudaError_t launch_lanczos_axpy(const double2 *vprev, double2 *r, int64_t nc, in
 cudaError_t launch_dot(const double2 *a, const double2 *b, int64_t nc, double2 *partial,
                        double2 *result, cudaStream_t st);
 
+// The whole Lanczos of a small space as one persistent launch (small.cu), for
+// real momentum-block integrals on spaces that the direct form covers: V (lm x
+// nc, V[0] the start vector), r (nc), s.alpha / s.beta / s.iters bit for bit as
+// the launch sequence leaves them (s.iters preset to lm), work of
+// small_lanczos_bytes. cudaErrorCooperativeLaunchTooLarge: cannot run here,
+// nothing was enqueued.
+constexpr uint32_t kSmallMaxRows = 16384;
+constexpr int kSmallMinSteps = 8;
+bool small_lanczos_fits(const Space &sp, int lm);
+size_t small_lanczos_bytes(const Space &sp, int lm);
+cudaError_t launch_small_lanczos(const Space &sp, const SpaceTables &tb, const PairOp &op, double2 *V, int lm,
+                                 double tol, double2 *r, LanczosState s, void *work, int device, cudaStream_t st);
+
 // Row-shard primitives of a sharded Lanczos (n rows of this rank; scalars on the
 // device; every kernel returns at entry once *done != 0). The caller sums the
 // per-rank results (dot, coef, norm2) over the ranks between the calls.

@@ -23,6 +23,7 @@ struct DevPairOp {
     double2 *hblk = nullptr;   // momentum-block form (nullptr when Ht couples different q+l)
     int nhblk = 0;
     std::vector<double2> hblk_h;   // host copy of hblk
+    bool real = false;             // the block values and the diagonal of Ho are real
     std::vector<double> contact;   // outer-product factors u[P] | w[P] of the blocks (empty: not of that form)
     int create_form = 0;
     int *status = nullptr;     // the space's device status word (not owned)
@@ -82,9 +83,9 @@ struct mcpi_space_s {
     uint32_t mr_lo = 0, mr_hi = 0;
     uint32_t *d_mr = nullptr;
     // grow-only workspaces kept between calls: Krylov basis of mcpi_ground,
-    // state block and residual of mcpi_lanczos
-    void *d_basis = nullptr, *d_lzblk = nullptr, *d_lzr = nullptr;
-    size_t basis_cap = 0, lzblk_cap = 0, lzr_cap = 0;
+    // state block and residual of mcpi_lanczos, lists and vectors of its one-launch form
+    void *d_basis = nullptr, *d_lzblk = nullptr, *d_lzr = nullptr, *d_small = nullptr;
+    size_t basis_cap = 0, lzblk_cap = 0, lzr_cap = 0, small_cap = 0;
     uint64_t *d_occ = nullptr;       // packed occupations of the space's rows (built by mcpi_set_integrals)
     uint64_t *d_occ2 = nullptr;      // the same for the (N-2)-particle space
     uint64_t *d_occ1 = nullptr;      // the same for the (N-1)-particle space (first rho1 call)
