@@ -19,6 +19,7 @@
 // a second kernel sums them in a fixed order and scatters them into the
 // reference layout, so the result is deterministic run to run.
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "fock.cuh"
 #include "kernels.h"
 #include "mbarrier.cuh"
@@ -497,16 +498,206 @@ __global__ void __launch_bounds__(DmmaGram<M, SAME>::THREADS, 1)
 
 // rho1 (and the transition rho1): G[a][b] = sum_h conj(Dphi[a][h]) Dpsi[b][h] over
 // the N-1 space with D[l][h] = sqrt(u_l+1) x[index(h + e_l)]. Only M columns, so
-// the Gram kernel above would keep one 4x4 block per thread busy (9 threads of
-// 256 at M = 10). Here a tile is kTile1 hole configurations, one per thread
-// (one decode each); the product gives every thread one entry (a, b) (a <= b
-// when phi = psi) and one of S interleaved subsets of the tile's
-// configurations; the subsets are summed in a fixed order at the end, so the
-// per-CTA partials (same layout as k_gram's) are deterministic.
+// a hole configuration's values fit one thread's registers: a lane takes one
+// configuration, gathers its M values and adds its products to accumulators
+// that it keeps for the whole launch; the entries (a <= b when phi = psi) are
+// split over the NS warps of a group, which read the same 32 configurations
+// (the second read hits L1). The next configurations' values are on their way
+// while the products of the current ones run. Lanes, then the block's groups,
+// are summed in a fixed order at the end, so the partials are deterministic.
+// Bound by the gathers through L1 (8 wavefronts per warp request) and the
+// FP64 pipe (4 multiply-adds per entry and configuration: 15 us at N=16, M=10).
+// Before, every entry read both its factors from shared memory for each
+// configuration (2 x 16 bytes per 4 multiply-adds, 63 us of shared-memory
+// bandwidth alone at N=16, M=10). Measured with the finish, N=16 and N=20, M=10:
+// 156 -> 60 us and 706 -> 289 us; two states 255 -> 112 us and 1213 -> 562 us.
+constexpr int kRho1Warps = 8;
+// Up to these M (us at the sizes N, M; this kernel / k_rho1_smem, finish included):
+// one state M=15 N=8 25 / 50, M=16 N=8 45 either way and 27 / 16 at N=6; two
+// states M=10 N=16 112 / 212, M=11 N=12 140 / 90, M=12 N=10 111 / 45.
+constexpr int kRho1MaxM = 15;        // rho1 of one state
+constexpr int kRho1MaxMTrans = 10;   // transition rho1
+
+template <int M, bool SAME>
+struct Rho1 {
+    static constexpr int E = SAME ? M * (M + 1) / 2 : M * M;   // entries
+    // warps that share the entries, so that the accumulators (4 registers each)
+    // and the values of two tiles fit a thread
+    static constexpr int MOST = SAME ? 30 : 25;
+    static constexpr int NS = E <= MOST ? 1 : E <= 2 * MOST ? 2 : E <= 4 * MOST ? 4 : 8;
+    static constexpr int GROUPS = kRho1Warps / NS;
+    // the next values are fetched ahead while they fit the registers
+    static constexpr bool AHEAD = M <= 12;
+    // one state: entries in row order, cut into NS ranges; two states: RS x CS
+    // rectangles (fewest values per entry)
+    static constexpr int CS = SAME ? 1 : NS >= 4 ? 2 : 1, RS = NS / CS;
+    static constexpr __host__ __device__ int first(int part) { return part * E / NS; }
+    static constexpr __host__ __device__ int row_of(int e)
+    {
+        int a = 0;
+        while (e >= M - a) {
+            e -= M - a;
+            ++a;
+        }
+        return a;
+    }
+    // rows [a0, a1) and columns [b0, M or b1) that a part reads
+    static constexpr __host__ __device__ int a0(int p) { return SAME ? row_of(first(p)) : p / CS * M / RS; }
+    static constexpr __host__ __device__ int a1(int p)
+    {
+        return SAME ? row_of(first(p + 1) - 1) + 1 : (p / CS + 1) * M / RS;
+    }
+    static constexpr __host__ __device__ int b0(int p) { return SAME ? a0(p) : p % CS * M / CS; }
+    static constexpr __host__ __device__ int b1(int p) { return SAME ? M : (p % CS + 1) * M / CS; }
+    static constexpr __host__ __device__ int count(int p)
+    {
+        return SAME ? first(p + 1) - first(p) : (a1(p) - a0(p)) * (b1(p) - b0(p));
+    }
+};
+
+// The entries of part PART over the tiles of 32 configurations tile0, tile0 +
+// step, ..; entry (a, b)'s sum over lanes to out[a * M + b].
+template <int M, bool SAME, int PART>
+__device__ __forceinline__ void rho1_part(const Space &sp, const SpaceTables &tb, const uint32_t *W,
+                                          const double *sq, const double2 *__restrict__ phi,
+                                          const double2 *__restrict__ psi, uint32_t tile0, uint32_t step,
+                                          double2 *out)
+{
+    using R = Rho1<M, SAME>;
+    constexpr int NE = R::count(PART), A0 = R::a0(PART), A1 = R::a1(PART), B0 = R::b0(PART), B1 = R::b1(PART);
+    constexpr int E0 = SAME ? R::first(PART) - A0 * M + A0 * (A0 - 1) / 2 : 0;   // entries of row A0 before this part's
+    constexpr int NZ = SAME ? 1 : A1 - A0;
+    const int lane = threadIdx.x & 31, ws = sp.wstride;
+    const uint32_t nh = sp.nc1, ntiles = (nh + 31) / 32;
+    double2 acc[NE];
+#pragma unroll
+    for (int x = 0; x < NE; ++x) acc[x] = make_double2(0.0, 0.0);
+    double2 y[B1 - B0], z[NZ];   // psi of columns B0 .., phi of rows A0 ..
+    double fy[B1 - B0], fz[NZ];  // their factors sqrt(u_l + 1)
+    // the packed occupations are read one tile further ahead than the values:
+    // their loads would otherwise add a second L2 latency to every tile
+    uint64_t word = 0;
+    auto fetch_word = [&](uint32_t tile) {
+        const uint32_t h = tile * 32 + lane;
+        if (tb.occ1) word = tb.occ1[h < nh ? h : 0u];
+    };
+    auto fetch = [&](uint32_t tile) {
+        const uint32_t h = tile * 32 + lane;
+        const bool in = h < nh;
+        int u[M], Q[M];
+        if (tb.occ1)
+            occupations<M>(&word, tb.occ_bits, 0u, sp.N - 1, nh, W, ws, u, Q);
+        else
+            decode<M>(in ? h : 0u, sp.N - 1, nh, W, ws, u, Q);
+        if (tile + step < ntiles) fetch_word(tile + step);
+        // index(h + e_l) = base + sum_{i<l} W_i(Q_i + 1) - W_i(Q_i), base = index of h + e_0
+        uint32_t d[M], hi = 0;
+        d[0] = 0;
+#pragma unroll
+        for (int t = 1; t < M; ++t) {
+            const uint32_t w1 = W[(t - 1) * ws + Q[t - 1] + 1];
+            hi += w1;
+            d[t] = d[t - 1] + (w1 - W[(t - 1) * ws + Q[t - 1]]);
+        }
+        const uint32_t base = sp.nc - 1u - hi;
+#pragma unroll
+        for (int l = B0; l < B1; ++l) {
+            y[l - B0] = __ldg(psi + (base + d[l]));
+            fy[l - B0] = in ? sq[u[l] + 1] : 0.0;
+        }
+        if constexpr (!SAME) {
+#pragma unroll
+            for (int l = A0; l < A1; ++l) {
+                z[l - A0] = __ldg(phi + (base + d[l]));
+                fz[l - A0] = in ? sq[u[l] + 1] : 0.0;
+            }
+        }
+    };
+    if (tile0 < ntiles) fetch_word(tile0);
+    if (R::AHEAD && tile0 < ntiles) fetch(tile0);
+    for (uint32_t tile = tile0; tile < ntiles; tile += step) {
+        if (!R::AHEAD) fetch(tile);
+        double2 p[B1 - B0], q[NZ];
+#pragma unroll
+        for (int l = 0; l < B1 - B0; ++l) p[l] = make_double2(fy[l] * y[l].x, fy[l] * y[l].y);
+        if constexpr (!SAME) {
+#pragma unroll
+            for (int l = 0; l < NZ; ++l) q[l] = make_double2(fz[l] * z[l].x, fz[l] * z[l].y);
+        }
+        if (R::AHEAD && tile + step < ntiles) fetch(tile + step);
+        int e = -E0;
+#pragma unroll
+        for (int a = A0; a < A1; ++a)
+#pragma unroll
+            for (int b = SAME ? a : B0; b < B1; ++b) {
+                if (e >= 0 && e < NE) cfma_conj(acc[e], SAME ? p[a - B0] : q[a - A0], p[b - B0]);
+                ++e;
+            }
+    }
+    int e = -E0;
+#pragma unroll
+    for (int a = A0; a < A1; ++a)
+#pragma unroll
+        for (int b = SAME ? a : B0; b < B1; ++b) {
+            if (e >= 0 && e < NE) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) {
+                    acc[e].x += __shfl_down_sync(0xffffffffu, acc[e].x, o);
+                    acc[e].y += __shfl_down_sync(0xffffffffu, acc[e].y, o);
+                }
+                if (lane == 0) out[a * M + b] = acc[e];
+            }
+            ++e;
+        }
+}
+
+template <int M, bool SAME>
+__global__ void __launch_bounds__(kRho1Warps * 32, 1)
+    k_rho1(Space sp, SpaceTables tb, const double2 *__restrict__ phi, const double2 *__restrict__ psi,
+           double2 *__restrict__ partial)
+{
+    using R = Rho1<M, SAME>;
+    __shared__ double2 red[R::GROUPS][M * M];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *sq = reinterpret_cast<double *>(smem_raw);
+    uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);
+    for (int x = threadIdx.x; x < (M - 1) * sp.wstride; x += blockDim.x) W[x] = tb.W[x];
+    for (int x = threadIdx.x; x < sp.wstride; x += blockDim.x) sq[x] = tb.sq[x];
+    __syncthreads();
+    const int warp = threadIdx.x / 32, grp = warp / R::NS;
+    const uint32_t tile0 = blockIdx.x * R::GROUPS + grp, step = gridDim.x * R::GROUPS;
+    switch (warp % R::NS) {   // the part as a template argument: its accumulators are registers
+#define MCPI_PART(p)                                                                                       \
+    case p:                                                                                                \
+        if constexpr (p < R::NS) rho1_part<M, SAME, p>(sp, tb, W, sq, phi, psi, tile0, step, red[grp]); \
+        break;
+        MCPI_PART(0) MCPI_PART(1) MCPI_PART(2) MCPI_PART(3) MCPI_PART(4) MCPI_PART(5) MCPI_PART(6) MCPI_PART(7)
+#undef MCPI_PART
+    default: break;
+    }
+    __syncthreads();
+    double2 *out = partial + (size_t)blockIdx.x * M * M;
+    for (int e = threadIdx.x; e < M * M; e += blockDim.x) {
+        if (SAME && e / M > e % M) continue;
+        double2 g = red[0][e];
+#pragma unroll
+        for (int k = 1; k < R::GROUPS; ++k) {
+            g.x += red[k][e].x;
+            g.y += red[k][e].y;
+        }
+        out[e] = g;
+    }
+}
+
+// The same for the largest M (kRho1MaxM), where eight parts' unrolled code no
+// longer fits the instruction cache and the values no longer fit the registers:
+// a tile is kTile1 hole configurations, one per thread, staged in shared memory;
+// every thread takes one entry (a, b) (a <= b when phi = psi) and one of S
+// interleaved subsets of the tile's configurations, summed in a fixed order.
 constexpr int kTile1 = 256;
 
 template <int M, bool SAME>
-__global__ void __launch_bounds__(kThreads) k_rho1(Space sp, SpaceTables tb, const double2 *__restrict__ phi,
+__global__ void __launch_bounds__(kThreads) k_rho1_smem(Space sp, SpaceTables tb, const double2 *__restrict__ phi,
                                                    const double2 *__restrict__ psi,
                                                    double2 *__restrict__ partial)
 {
@@ -587,42 +778,76 @@ __global__ void __launch_bounds__(kThreads) k_rho1(Space sp, SpaceTables tb, con
         }
         double2 *out = partial + (size_t)blockIdx.x * M * M;
         out[a * M + b] = g;
-        if (SAME && a != b) out[b * M + a] = make_double2(g.x, -g.y);
     }
 }
 
-// Sums the per-CTA partials in block order and writes the reference layout.
-// HERM 1: the partials hold only the blocks of k_gram<.., SAME = true> (entry
-// (a, b) with a mod NB <= b mod NB); HERM 2: only the tiles of
-// k_gram_dmma<.., SAME = true> (entry (a, b) with b / 8 >= 2 (a / 16)). The
-// rest is the conjugate of the entry (b, a), which is then held.
+// Entries of the Gram matrix that the partials hold, by the kernel that wrote
+// them: all (HERM 0), the blocks of k_gram<.., SAME = true> (1), the tiles of
+// k_gram_dmma<.., SAME = true> (2), the upper triangle of k_rho1<.., true> (3).
+template <int HERM>
+__device__ __forceinline__ bool gram_held(int a, int b, int NB)
+{
+    return HERM == 1 ? a % NB <= b % NB : HERM == 2 ? b / 8 >= 2 * (a / 16) : HERM == 3 ? a <= b : true;
+}
+
+// Pair index -> (k, s), k <= s.
+__device__ __forceinline__ void pair_of(int p, int M, int &k, int &s)
+{
+    k = 0;
+    while (p >= M - k) {
+        p -= M - k;
+        ++k;
+    }
+    s = k + p;
+}
+
+// Sums the per-block partials in a fixed order and writes the reference layout:
+// a block takes 32 entries, its 32 warps every 32nd partial each (coalesced, all
+// loads in flight), then one warp per entry adds the 32 sums and writes the
+// entry, its permutations and, where that is not held itself, its conjugate.
+// (One thread per output, adding the partials one after the other, took 41 us
+// after rho1 and 30 us after rho2 at M=10; this takes 3 to 4 us.)
 template <int M, int ORDER, int HERM = 0>
-__global__ void k_gram_finish(const double2 *__restrict__ partial, int nblocks,
-                              double2 *__restrict__ out)
+__global__ void __launch_bounds__(1024) k_gram_finish(const double2 *__restrict__ partial, int nblocks,
+                                                      double2 *__restrict__ out)
 {
     using C = Cols<M, ORDER>;
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int a, b;
-    if (ORDER == 1) {
-        if (x >= M * M) return;
-        a = x / M;              // rho1[k*M + l] = G[k][l]
-        b = x % M;
+    __shared__ double2 red[32][33];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    {
+        const int e = blockIdx.x * 32 + lane;
+        double2 acc = make_double2(0.0, 0.0);
+        if (e < C::K * C::K && gram_held<HERM>(e / C::K, e % C::K, C::NB)) {
+#pragma unroll 5
+            for (int blk = warp; blk < nblocks; blk += 32) {
+                const double2 p = partial[(size_t)blk * C::K * C::K + e];
+                acc.x += p.x;
+                acc.y += p.y;
+            }
+        }
+        red[warp][lane] = acc;
+    }
+    __syncthreads();
+    const int e = blockIdx.x * 32 + warp, a = e / C::K, b = e % C::K;
+    if (e >= C::K * C::K || !gram_held<HERM>(a, b, C::NB)) return;
+    double2 g = red[lane][warp];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        g.x += __shfl_xor_sync(0xffffffffu, g.x, o);
+        g.y += __shfl_xor_sync(0xffffffffu, g.y, o);
+    }
+    const bool mirror = HERM != 0 && !gram_held<HERM>(b, a, C::NB);
+    if constexpr (ORDER == 1) {
+        if (lane == 0) out[a * M + b] = g;   // rho1[k*M + l] = G[k][l]
+        if (lane == 1 && mirror) out[b * M + a] = make_double2(g.x, -g.y);
     } else {
-        if (x >= M * M * M * M) return;
-        const int k = x % M, s = (x / M) % M, q = (x / (M * M)) % M, l = x / (M * M * M);
-        a = k <= s ? pair_index(k, s, M) : pair_index(s, k, M);
-        b = q <= l ? pair_index(q, l, M) : pair_index(l, q, M);
+        int k, s, q, l;
+        pair_of(a, M, k, s);
+        pair_of(b, M, q, l);
+        const int x = lane & 1 ? s : k, y = lane & 1 ? k : s, z = lane & 2 ? l : q, w = lane & 2 ? q : l;
+        if (lane < 4) out[x + y * M + z * M * M + w * M * M * M] = g;
+        if (lane >= 4 && lane < 8 && mirror) out[z + w * M + x * M * M + y * M * M * M] = make_double2(g.x, -g.y);
     }
-    const bool mirror = HERM == 1 ? (a % C::NB) > (b % C::NB) : HERM == 2 ? (b / 8) < 2 * (a / 16) : false;
-    const int e = mirror ? b * C::K + a : a * C::K + b;
-    double2 acc = make_double2(0.0, 0.0);
-    for (int blk = 0; blk < nblocks; ++blk) {
-        const double2 p = partial[(size_t)blk * C::K * C::K + e];
-        acc.x += p.x;
-        acc.y += p.y;
-    }
-    if (mirror) acc.y = -acc.y;
-    out[x] = acc;
 }
 
 template <int M, int ORDER>
@@ -632,28 +857,36 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
 {
     using C = Cols<M, ORDER>;
     const bool same = (phi == psi);
+    constexpr unsigned finish = (C::K * C::K + 31) / 32;
     if constexpr (ORDER == 1) {
-        const size_t smem = sizeof(double2) * ((same ? 1 : 2) * (size_t)M * (kTile1 + 1) + kThreads) +
-                            sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
-        const unsigned ntiles = (sp.nc1 + kTile1 - 1) / kTile1;
-        const unsigned gx = ntiles < (unsigned)kGramBlocks ? (ntiles ? ntiles : 1) : kGramBlocks;
-        cudaError_t e;
-        if (same) {
-            e = cudaFuncSetAttribute(k_rho1<M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-            k_rho1<M, true><<<gx, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
-        } else {
-            e = cudaFuncSetAttribute(k_rho1<M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return e;
-            k_rho1<M, false><<<gx, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
-        }
-        k_gram_finish<M, 1><<<(M * M + 255) / 256, 256, 0, st>>>(partial, gx, out);
+        const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
+        auto run = [&](auto state) -> cudaError_t {
+            constexpr bool SAME = decltype(state)::value;
+            if constexpr (M <= (SAME ? kRho1MaxM : kRho1MaxMTrans)) {
+                constexpr unsigned per = 32 * Rho1<M, SAME>::GROUPS;   // configurations per pass of a block
+                const unsigned need = (sp.nc1 + per - 1) / per;
+                const unsigned gx = need < (unsigned)kDmmaBlocks ? (need ? need : 1) : kDmmaBlocks;
+                k_rho1<M, SAME><<<gx, kRho1Warps * 32, tab, st>>>(sp, tb, phi, psi, partial);
+                k_gram_finish<M, 1, SAME ? 3 : 0><<<finish, 1024, 0, st>>>(partial, gx, out);
+            } else {
+                const size_t smem = sizeof(double2) * ((SAME ? 1 : 2) * (size_t)M * (kTile1 + 1) + kThreads) + tab;
+                const unsigned ntiles = (sp.nc1 + kTile1 - 1) / kTile1;
+                const unsigned gx = ntiles < (unsigned)kGramBlocks ? (ntiles ? ntiles : 1) : kGramBlocks;
+                const cudaError_t e = cudaFuncSetAttribute(k_rho1_smem<M, SAME>,
+                                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                if (e != cudaSuccess) return e;
+                k_rho1_smem<M, SAME><<<gx, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
+                k_gram_finish<M, 1, SAME ? 3 : 0><<<finish, 1024, 0, st>>>(partial, gx, out);
+            }
+            return cudaSuccess;
+        };
+        const cudaError_t e = same ? run(std::true_type{}) : run(std::false_type{});
+        if (e != cudaSuccess) return e;
         return cudaGetLastError();
     }
     if constexpr (ORDER == 2 && M >= 2 && M <= kDmmaMaxM) {
         // FP64 tensor cores (the transition form up to kDmmaMaxMTrans), when the
         // stages and the space's tables fit the block's shared memory
-        const int nout = M * M * M * M;
         int dev = 0, optin = 0;
         cudaError_t qe = cudaGetDevice(&dev);
         if (qe == cudaSuccess) qe = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -667,7 +900,7 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
             if (e != cudaSuccess) return e;
             k_gram_dmma<M, true><<<gx, Dm::THREADS, sm, st>>>(sp, tb, phi, psi, partial, status, wait_cycles,
                                                                test_stall);
-            k_gram_finish<M, 2, 2><<<(nout + 255) / 256, 256, 0, st>>>(partial, gx, out);
+            k_gram_finish<M, 2, 2><<<finish, 1024, 0, st>>>(partial, gx, out);
             return cudaGetLastError();
         }
         if constexpr (M <= kDmmaMaxMTrans) {
@@ -680,7 +913,7 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
             if (e != cudaSuccess) return e;
             k_gram_dmma<M, false><<<gx, Dm::THREADS, sm, st>>>(sp, tb, phi, psi, partial, status, wait_cycles,
                                                                 test_stall);
-            k_gram_finish<M, 2, 0><<<(nout + 255) / 256, 256, 0, st>>>(partial, gx, out);
+            k_gram_finish<M, 2, 0><<<finish, 1024, 0, st>>>(partial, gx, out);
             return cudaGetLastError();
             }
         }
@@ -703,11 +936,10 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
         if (e != cudaSuccess) return e;
         k_gram<M, ORDER, false><<<grid, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
     }
-    const int nout = ORDER == 1 ? M * M : M * M * M * M;
     if (same)
-        k_gram_finish<M, ORDER, 1><<<(nout + 255) / 256, 256, 0, st>>>(partial, gx, out);
+        k_gram_finish<M, ORDER, 1><<<finish, 1024, 0, st>>>(partial, gx, out);
     else
-        k_gram_finish<M, ORDER, 0><<<(nout + 255) / 256, 256, 0, st>>>(partial, gx, out);
+        k_gram_finish<M, ORDER, 0><<<finish, 1024, 0, st>>>(partial, gx, out);
     return cudaGetLastError();
 }
 
