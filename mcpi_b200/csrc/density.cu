@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(DmmaGram<M, SAME>::THREADS, 1)
             mbar_init(full + b, D::GT);
             mbar_init(empty + b, kDmmaPW);
         }
+    pdl_wait();
     __syncthreads();
 
     const uint32_t nh = sp.nc2;
@@ -663,6 +664,7 @@ __global__ void __launch_bounds__(kRho1Warps * 32, 1)
     uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);
     for (int x = threadIdx.x; x < (M - 1) * sp.wstride; x += blockDim.x) W[x] = tb.W[x];
     for (int x = threadIdx.x; x < sp.wstride; x += blockDim.x) sq[x] = tb.sq[x];
+    pdl_wait();
     __syncthreads();
     const int warp = threadIdx.x / 32, grp = warp / R::NS;
     const uint32_t tile0 = blockIdx.x * R::GROUPS + grp, step = gridDim.x * R::GROUPS;
@@ -814,6 +816,7 @@ __global__ void __launch_bounds__(1024) k_gram_finish(const double2 *__restrict_
     using C = Cols<M, ORDER>;
     __shared__ double2 red[32][33];
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    pdl_wait();
     {
         const int e = blockIdx.x * 32 + lane;
         double2 acc = make_double2(0.0, 0.0);
@@ -866,8 +869,9 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
                 constexpr unsigned per = 32 * Rho1<M, SAME>::GROUPS;   // configurations per pass of a block
                 const unsigned need = (sp.nc1 + per - 1) / per;
                 const unsigned gx = need < (unsigned)kDmmaBlocks ? (need ? need : 1) : kDmmaBlocks;
-                k_rho1<M, SAME><<<gx, kRho1Warps * 32, tab, st>>>(sp, tb, phi, psi, partial);
-                k_gram_finish<M, 1, SAME ? 3 : 0><<<finish, 1024, 0, st>>>(partial, gx, out);
+                cudaError_t e = launch_pdl(k_rho1<M, SAME>, gx, kRho1Warps * 32, tab, st, sp, tb, phi, psi, partial);
+                if (e != cudaSuccess) return e;
+                return launch_pdl(k_gram_finish<M, 1, SAME ? 3 : 0>, finish, 1024, 0, st, partial, (int)gx, out);
             } else {
                 const size_t smem = sizeof(double2) * ((SAME ? 1 : 2) * (size_t)M * (kTile1 + 1) + kThreads) + tab;
                 const unsigned ntiles = (sp.nc1 + kTile1 - 1) / kTile1;
@@ -876,9 +880,8 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) return e;
                 k_rho1_smem<M, SAME><<<gx, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
-                k_gram_finish<M, 1, SAME ? 3 : 0><<<finish, 1024, 0, st>>>(partial, gx, out);
+                return launch_pdl(k_gram_finish<M, 1, SAME ? 3 : 0>, finish, 1024, 0, st, partial, (int)gx, out);
             }
-            return cudaSuccess;
         };
         const cudaError_t e = same ? run(std::true_type{}) : run(std::false_type{});
         if (e != cudaSuccess) return e;
@@ -898,10 +901,10 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
             const size_t sm = Dm::smem(sp.wstride);
             cudaError_t e = cudaFuncSetAttribute(k_gram_dmma<M, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             if (e != cudaSuccess) return e;
-            k_gram_dmma<M, true><<<gx, Dm::THREADS, sm, st>>>(sp, tb, phi, psi, partial, status, wait_cycles,
-                                                               test_stall);
-            k_gram_finish<M, 2, 2><<<finish, 1024, 0, st>>>(partial, gx, out);
-            return cudaGetLastError();
+            e = launch_pdl(k_gram_dmma<M, true>, gx, Dm::THREADS, sm, st, sp, tb, phi, psi, partial, status, wait_cycles,
+                           test_stall);
+            if (e != cudaSuccess) return e;
+            return launch_pdl(k_gram_finish<M, 2, 2>, finish, 1024, 0, st, partial, (int)gx, out);
         }
         if constexpr (M <= kDmmaMaxMTrans) {
             if (!same && DmmaGram<M, false>::smem(sp.wstride) <= (size_t)optin) {
@@ -911,10 +914,10 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
             const size_t sm = Dm::smem(sp.wstride);
             cudaError_t e = cudaFuncSetAttribute(k_gram_dmma<M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             if (e != cudaSuccess) return e;
-            k_gram_dmma<M, false><<<gx, Dm::THREADS, sm, st>>>(sp, tb, phi, psi, partial, status, wait_cycles,
-                                                                test_stall);
-            k_gram_finish<M, 2, 0><<<finish, 1024, 0, st>>>(partial, gx, out);
-            return cudaGetLastError();
+            e = launch_pdl(k_gram_dmma<M, false>, gx, Dm::THREADS, sm, st, sp, tb, phi, psi, partial, status, wait_cycles,
+                           test_stall);
+            if (e != cudaSuccess) return e;
+            return launch_pdl(k_gram_finish<M, 2, 0>, finish, 1024, 0, st, partial, (int)gx, out);
             }
         }
     }
@@ -937,9 +940,9 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
         k_gram<M, ORDER, false><<<grid, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
     }
     if (same)
-        k_gram_finish<M, ORDER, 1><<<finish, 1024, 0, st>>>(partial, gx, out);
+        return launch_pdl(k_gram_finish<M, ORDER, 1>, finish, 1024, 0, st, partial, (int)gx, out);
     else
-        k_gram_finish<M, ORDER, 0><<<finish, 1024, 0, st>>>(partial, gx, out);
+        return launch_pdl(k_gram_finish<M, ORDER, 0>, finish, 1024, 0, st, partial, (int)gx, out);
     return cudaGetLastError();
 }
 

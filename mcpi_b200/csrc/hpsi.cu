@@ -446,6 +446,7 @@ __global__ void __launch_bounds__(kTW, 1)
             mbar_init(full + b, kGM);
             mbar_init(empty + b, kProdThreads / 32);
         }
+    pdl_wait();
     __syncthreads();
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -730,6 +731,7 @@ __device__ __forceinline__ void annihilate_momentum_body(const Space &sp, const 
     if (!PARAM)
         for (int x = threadIdx.x; x < nh; x += blockDim.x) hs[x] = hblk[x];
     const double2 *hv = PARAM ? hblk : hs;
+    pdl_wait();
     __syncthreads();
 
     const uint32_t m = m0 + block * kT2 + threadIdx.x;
@@ -968,6 +970,7 @@ __device__ __forceinline__ void create_smem_body(const Space &sp, const SpaceTab
     uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);   // (M-1) x wstride
     load_tables(sp, tb, W, sq);
     if (threadIdx.x < M) hd[threadIdx.x] = hdiag[threadIdx.x];
+    pdl_wait();
     __syncthreads();
 
     const uint32_t i = row0 + block * kTC + threadIdx.x;   // rows [row0, row1) -> out[i - row0]
@@ -1168,6 +1171,7 @@ __global__ void __launch_bounds__(kTC, 3)
     uint32_t *W = reinterpret_cast<uint32_t *>(sqp + ws * ws);
     uint32_t *FS = W + (M - 1) * ws, *GS = FS + M * kTC;
     direct_tables<M>(ws, tb.W, tb.sq, hdiag, hd, sqp, W);
+    pdl_wait();
     __syncthreads();
     const uint32_t i = row0 + blockIdx.x * kTC + threadIdx.x;   // rows [row0, row1) -> out[i - row0]
     if (i >= row1) return;
@@ -1190,8 +1194,7 @@ cudaError_t launch_direct(const Space &sp, const SpaceTables &tb, const MomBlock
         if (e != cudaSuccess) return e;
     }
     const unsigned grid = (row1 - row0 + kTC - 1) / kTC;
-    k_hpsi_direct<M, REAL, R, SMEM_D><<<grid, kTC, smem, st>>>(sp, tb, hp, hdiag, psi, out, row0, row1);
-    return cudaGetLastError();
+    return launch_pdl(k_hpsi_direct<M, REAL, R, SMEM_D>, grid, kTC, smem, st, sp, tb, hp, hdiag, psi, out, row0, row1);
 }
 
 template <int M>
@@ -1234,6 +1237,7 @@ __global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb
     double *sq = reinterpret_cast<double *>(smem_raw);            // wstride
     uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);  // (M-1) x wstride
     load_tables(sp, tb, W, sq);
+    pdl_wait();
     __syncthreads();
     const uint32_t m = m0 + blockIdx.x * kT2 + threadIdx.x;
     if (m >= m1) return;
@@ -1295,6 +1299,7 @@ __global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables
     uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);   // (M-1) x wstride
     load_tables(sp, tb, W, sq);
     if (threadIdx.x < M) hd[threadIdx.x] = hdiag[threadIdx.x];
+    pdl_wait();
     __syncthreads();
     // from the top rows down: their S entries were written last, some are still in L2
     const uint32_t i = row0 + (gridDim.x - 1 - blockIdx.x) * kTC + threadIdx.x;
@@ -1371,20 +1376,21 @@ cudaError_t contact_apply_m(const Space &sp, const SpaceTables &tb, const PairOp
     }
     const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
     if (m1 > sp.nc2) m1 = sp.nc2;
+    cudaError_t e = cudaSuccess;
     if ((stages & 1) && m1 > m0)
-        k_contact_sum<M><<<(m1 - m0 + kT2 - 1) / kT2, kT2, tab, st>>>(sp, tb, cv, psi, S, m0, m1);
+        e = launch_pdl(k_contact_sum<M>, (m1 - m0 + kT2 - 1) / kT2, kT2, tab, st, sp, tb, cv, psi, S, m0, m1);
     if ((stages & 2) && row1 > row0) {
         const size_t sm = (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + ((M * kTC + 15) & ~15) +
                           sizeof(double2) * M + tab;
         if (sm > 48 * 1024) {
-            const cudaError_t e = cudaFuncSetAttribute(k_contact_create<M>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            if (e != cudaSuccess) return e;
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(k_contact_create<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         }
-        k_contact_create<M><<<(row1 - row0 + kTC - 1) / kTC, kTC, sm, st>>>(sp, tb, cv, op.hdiag, psi, S, out, row0,
-                                                                          row1);
+        if (e == cudaSuccess)
+            e = launch_pdl(k_contact_create<M>, (row1 - row0 + kTC - 1) / kTC, kTC, sm, st, sp, tb, cv, op.hdiag, psi,
+                           S, out, row0, row1);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace
@@ -1830,7 +1836,9 @@ cudaError_t apply_h_m(const Space &sp, const SpaceTables &tb, const PairOp &op, 
         if (g1 && op.hblk_host && op.nhblk == mom_values<M>()) {
             MomBlocks<M> hp;
             for (int x = 0; x < mom_values<M>(); ++x) hp.v[x] = op.hblk_host[x];
-            k_pair_annihilate_momentum_p<M><<<g1, kT2, tab, st>>>(sp, tb, hp, psi, E, m0, m1);
+            if (const cudaError_t e = launch_pdl(k_pair_annihilate_momentum_p<M>, g1, kT2, tab, st, sp, tb, hp, psi, E, m0, m1);
+                e != cudaSuccess)
+                return e;
         } else if (g1) {
             const size_t smm = sizeof(double2) * op.nhblk + tab;
             k_pair_annihilate_momentum<M><<<g1, kT2, smm, st>>>(sp, tb, op.hblk, op.nhblk, psi, E, m0, m1);
@@ -1866,25 +1874,25 @@ cudaError_t apply_h_m(const Space &sp, const SpaceTables &tb, const PairOp &op, 
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smc2)) != cudaSuccess)
                     return e;
                 if (gw)
-                    k_pair_annihilate_gemm_ws<M, 2, true>
-                        <<<gw, kTW, smc2, st>>>(sp, tb, op.hdense, psi, E, ntiles, op.status,
-                                                                         op.wait_cycles, op.test_stall);
+                    e = launch_pdl(k_pair_annihilate_gemm_ws<M, 2, true>, gw, kTW, smc2, st, sp, tb, op.hdense, psi, E, ntiles,
+                                   op.status, op.wait_cycles, op.test_stall);
+                if (e != cudaSuccess) return e;
             } else if (smw3 <= (size_t)optin) {
                 if ((e = cudaFuncSetAttribute(k_pair_annihilate_gemm_ws<M, 3, false>,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw3)) != cudaSuccess)
                     return e;
                 if (gw)
-                    k_pair_annihilate_gemm_ws<M, 3, false>
-                        <<<gw, kTW, smw3, st>>>(sp, tb, op.hdense, psi, E, ntiles, op.status,
-                                                                         op.wait_cycles, op.test_stall);
+                    e = launch_pdl(k_pair_annihilate_gemm_ws<M, 3, false>, gw, kTW, smw3, st, sp, tb, op.hdense, psi, E, ntiles,
+                                   op.status, op.wait_cycles, op.test_stall);
+                if (e != cudaSuccess) return e;
             } else if (smw2 <= (size_t)optin) {
                 if ((e = cudaFuncSetAttribute(k_pair_annihilate_gemm_ws<M, 2, false>,
                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw2)) != cudaSuccess)
                     return e;
                 if (gw)
-                    k_pair_annihilate_gemm_ws<M, 2, false>
-                        <<<gw, kTW, smw2, st>>>(sp, tb, op.hdense, psi, E, ntiles, op.status,
-                                                                         op.wait_cycles, op.test_stall);
+                    e = launch_pdl(k_pair_annihilate_gemm_ws<M, 2, false>, gw, kTW, smw2, st, sp, tb, op.hdense, psi, E, ntiles,
+                                   op.status, op.wait_cycles, op.test_stall);
+                if (e != cudaSuccess) return e;
             } else {
                 const size_t smg = G::hbytes + G::dbytes + tab;
                 if ((e = cudaFuncSetAttribute(k_pair_annihilate_gemm<M>,
@@ -1915,7 +1923,7 @@ cudaError_t apply_h_m(const Space &sp, const SpaceTables &tb, const PairOp &op, 
             if (e != cudaSuccess) return e;
         }
         const unsigned g2 = (row1 - row0 + kTC - 1) / kTC;
-        if (g2) k_pair_create_smem<M><<<g2, kTC, sm2, st>>>(sp, tb, op, psi, E, out, row0, row1);
+        if (g2) return launch_pdl(k_pair_create_smem<M>, g2, kTC, sm2, st, sp, tb, op, psi, E, out, row0, row1);
     } else if (stages & 2) {
         if (row0 != 0 || row1 != sp.nc) return cudaErrorInvalidValue;   // row ranges: shared-table form only
         const size_t sm2 = sizeof(double2) * M + tab;

@@ -7,6 +7,41 @@
 
 namespace mcpi {
 
+// Programmatic dependent launch. A kernel launched with launch_pdl may start
+// while the last blocks of the kernel before it on the stream still run: its
+// launch latency and its prologue (tables into shared memory) overlap that
+// kernel's tail. Every thread of such a kernel calls pdl_wait() before it
+// touches anything that an earlier kernel may write or read -- all but the
+// space's constant tables and the operator's values, which the host has
+// finished uploading -- and nothing returns before it, so completion stays
+// transitive along the stream. The start is triggered by the earlier kernel's
+// blocks as they exit, not by an explicit trigger: triggered early, whole
+// chains of waiting kernels became resident and took the slots that spread the
+// next one over the SMs (Lanczos N=10, M=9: 7.8 ms without, 10.0 ms triggered
+// at entry, 5.8 ms after the wait, 5.4 ms at exit). Measured (B200): H.psi
+// N=9, M=13 49.8 -> 44.2 us, N=16, M=10 209 -> 198 us, general N=10, M=10 38.9 ->
+// 34.7 us; H.psi, its adjoint and both transition densities at N=8, M=8 59.6 ->
+// 52.5 us; 100 Lanczos steps N=12, M=8 8.0 -> 5.8 ms.
+#ifdef __CUDACC__
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A &...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
+
 // Fused H.psi (momentum-block form only). One persistent launch runs the
 // tiles of kernel 1 (producers: 256 (N-2)-configurations each, writing E) and
 // of kernel 2 (consumers: 256 rows each, reading E) in one interleaved order,

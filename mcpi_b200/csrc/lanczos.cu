@@ -69,6 +69,7 @@ __device__ __forceinline__ bool stopped(const int *done) { return done && *done;
 __global__ void k_dot_partial(const double2 *__restrict__ a, const double2 *__restrict__ b,
                               int64_t n, double2 *__restrict__ partial, const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     double2 acc = make_double2(0.0, 0.0);
     for (int64_t r = blockIdx.x * (int64_t)kThreads + threadIdx.x; r < n;
@@ -85,6 +86,7 @@ __global__ void k_dot_partial(const double2 *__restrict__ a, const double2 *__re
 __global__ void k_sum_partials(const double2 *__restrict__ partial, int n, double2 *out,
                                const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     double2 acc = make_double2(0.0, 0.0);
     // fixed assignment: thread t sums t, t+256, ... then a fixed-order block sum
@@ -101,6 +103,7 @@ __global__ void k_axpy_dot(const double2 *__restrict__ vprev, const double2 *__r
                            double2 *__restrict__ r, int64_t n, const double *beta_i,
                            double2 *__restrict__ partial, const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     const double b = *beta_i;
     double2 acc = make_double2(0.0, 0.0);
@@ -123,6 +126,7 @@ __global__ void k_axpy_dot(const double2 *__restrict__ vprev, const double2 *__r
 __global__ void k_axpy(const double2 *__restrict__ vprev, double2 *__restrict__ r, int64_t n,
                        const double *beta_i, const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     const double b = *beta_i;
     for (int64_t x = blockIdx.x * (int64_t)kThreads + threadIdx.x; x < n;
@@ -143,6 +147,7 @@ __global__ void __launch_bounds__(kThreads) k_multidot(const double2 *__restrict
                                                        double2 *__restrict__ partial,
                                                        const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     __shared__ double2 xs[kSlice];
     const int64_t r0 = (int64_t)blockIdx.x * kSlice;
@@ -173,6 +178,7 @@ __global__ void __launch_bounds__(kThreads) k_multidot(const double2 *__restrict
 __global__ void k_multidot_finish(const double2 *__restrict__ partial, int nblk, int nvec,
                                   double2 *__restrict__ coef, const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     const int j = blockIdx.x * (kThreads / 32) + threadIdx.x / 32, lane = threadIdx.x % 32;
     if (j >= nvec) return;
@@ -196,6 +202,7 @@ __global__ void __launch_bounds__(kThreads) k_update(const double2 *__restrict__
                                                      double2 *__restrict__ partial,
                                                      const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     extern __shared__ double2 cs[];
     for (int j = threadIdx.x; j < nvec; j += kThreads) cs[j] = coef[j];
@@ -235,6 +242,7 @@ __global__ void __launch_bounds__(kThreads) k_update(const double2 *__restrict__
 __global__ void k_beta(const double2 *__restrict__ partial, int n, int i, double tol,
                        double *beta, double *maxbeta, int *done, int *iters)
 {
+    pdl_wait();
     if (*done) return;
     double2 acc = make_double2(0.0, 0.0);
     for (int b = threadIdx.x; b < n; b += kThreads) acc.x += partial[b].x;
@@ -255,6 +263,7 @@ __global__ void k_beta(const double2 *__restrict__ partial, int n, int i, double
 __global__ void k_beta_total(const double *norm2, int i, double tol, double *beta, double *maxbeta, int *done,
                              int *iters)
 {
+    pdl_wait();
     if (*done || threadIdx.x != 0) return;
     const double bi = sqrt(*norm2);
     beta[i] = bi;
@@ -268,6 +277,7 @@ __global__ void k_beta_total(const double *norm2, int i, double tol, double *bet
 // *out = real part of sum_b partial[b] (b in order); one block.
 __global__ void k_sum_partials_re(const double2 *__restrict__ partial, int n, double *out, const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     double2 acc = make_double2(0.0, 0.0);
     for (int b = threadIdx.x; b < n; b += kThreads) acc.x += partial[b].x;
@@ -278,6 +288,7 @@ __global__ void k_sum_partials_re(const double2 *__restrict__ partial, int n, do
 __global__ void k_scale(const double2 *__restrict__ r, double2 *__restrict__ vnext, int64_t n,
                         const double *beta_i, const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     const double b = *beta_i;
     for (int64_t x = blockIdx.x * (int64_t)kThreads + threadIdx.x; x < n;
@@ -291,6 +302,7 @@ __global__ void k_scale(const double2 *__restrict__ r, double2 *__restrict__ vne
 __global__ void k_axpy_real(double2 *__restrict__ acc, const double2 *__restrict__ v, int64_t n,
                             const double *z, int first, const int *done)
 {
+    pdl_wait();
     if (stopped(done)) return;
     const double c = *z;
     for (int64_t x = blockIdx.x * (int64_t)kThreads + threadIdx.x; x < n;
@@ -308,6 +320,7 @@ __global__ void k_combine(const double2 *__restrict__ V, int nvec, int64_t n,
                           const double *__restrict__ z, double2 *__restrict__ out)
 {
     extern __shared__ double zs[];
+    pdl_wait();
     for (int j = threadIdx.x; j < nvec; j += kThreads) zs[j] = z[j];
     __syncthreads();
     for (int64_t x = blockIdx.x * (int64_t)kThreads + threadIdx.x; x < n;
@@ -346,8 +359,8 @@ cudaError_t launch_dot(const double2 *a, const double2 *b, int64_t nc, double2 *
                        double2 *result, cudaStream_t st)
 {
     const unsigned g = grid_for(nc);
-    k_dot_partial<<<g, kThreads, 0, st>>>(a, b, nc, partial, nullptr);
-    k_sum_partials<<<1, kThreads, 0, st>>>(partial, g, result, nullptr);
+    (void)launch_pdl(k_dot_partial, g, kThreads, 0, st, a, b, nc, partial, nullptr);
+    (void)launch_pdl(k_sum_partials, 1, kThreads, 0, st, partial, g, result, nullptr);
     return cudaGetLastError();
 }
 
@@ -360,23 +373,23 @@ cudaError_t launch_lanczos_start(const double2 *v0, const double2 *hv, double2 *
         cudaError_t e = cudaMemcpyAsync(r, hv, sizeof(double2) * nc, cudaMemcpyDeviceToDevice, st);
         if (e != cudaSuccess) return e;
     }
-    k_dot_partial<<<g, kThreads, 0, st>>>(v0, r, nc, s.partial, s.done);
-    k_sum_partials<<<1, kThreads, 0, st>>>(s.partial, g, s.alpha, s.done);
-    k_update<<<g, kThreads, 0, st>>>(nullptr, 0, nc, r, v0, s.alpha, nullptr, s.partial, s.done);
+    (void)launch_pdl(k_dot_partial, g, kThreads, 0, st, v0, r, nc, s.partial, s.done);
+    (void)launch_pdl(k_sum_partials, 1, kThreads, 0, st, s.partial, g, s.alpha, s.done);
+    (void)launch_pdl(k_update, g, kThreads, 0, st, nullptr, 0, nc, r, v0, s.alpha, nullptr, s.partial, s.done);
     return cudaGetLastError();
 }
 
 cudaError_t launch_lanczos_beta(int i, int lm, double tol, LanczosState s, cudaStream_t st)
 {
     (void)lm;
-    k_beta<<<1, kThreads, 0, st>>>(s.partial, s.nparts, i, tol, s.beta, s.maxbeta, s.done, s.iters);
+    (void)launch_pdl(k_beta, 1, kThreads, 0, st, s.partial, s.nparts, i, tol, s.beta, s.maxbeta, s.done, s.iters);
     return cudaGetLastError();
 }
 
 cudaError_t launch_lanczos_scale(const double2 *r, double2 *vnext, int64_t nc, int i,
                                  LanczosState s, cudaStream_t st)
 {
-    k_scale<<<grid_for(nc), kThreads, 0, st>>>(r, vnext, nc, s.beta + i, s.done);
+    (void)launch_pdl(k_scale, grid_for(nc), kThreads, 0, st, r, vnext, nc, s.beta + i, s.done);
     return cudaGetLastError();
 }
 
@@ -385,8 +398,8 @@ cudaError_t launch_lanczos_alpha(const double2 *vprev, const double2 *vcur, doub
                                  int64_t nc, int i, LanczosState s, cudaStream_t st)
 {
     const unsigned g = grid_for(nc);
-    k_axpy_dot<<<g, kThreads, 0, st>>>(vprev, vcur, r, nc, s.beta + i, s.partial, s.done);
-    k_sum_partials<<<1, kThreads, 0, st>>>(s.partial, g, s.alpha + i + 1, s.done);
+    (void)launch_pdl(k_axpy_dot, g, kThreads, 0, st, vprev, vcur, r, nc, s.beta + i, s.partial, s.done);
+    (void)launch_pdl(k_sum_partials, 1, kThreads, 0, st, s.partial, g, s.alpha + i + 1, s.done);
     return cudaGetLastError();
 }
 
@@ -396,10 +409,10 @@ cudaError_t launch_lanczos_reorth(const double2 *V, int nvec, double2 *r, int64_
 {
     const double2 *vcur = V + (size_t)(i + 1) * nc;
     const unsigned nblk = (unsigned)((nc + kSlice - 1) / kSlice);
-    k_multidot<<<nblk, kThreads, 0, st>>>(V, nvec, nc, r, vcur, s.alpha + i + 1, s.partial, s.done);
-    k_multidot_finish<<<(nvec + 7) / 8, kThreads, 0, st>>>(s.partial, nblk, nvec, s.coef, s.done);
+    (void)launch_pdl(k_multidot, nblk, kThreads, 0, st, V, nvec, nc, r, vcur, s.alpha + i + 1, s.partial, s.done);
+    (void)launch_pdl(k_multidot_finish, (nvec + 7) / 8, kThreads, 0, st, s.partial, nblk, nvec, s.coef, s.done);
     const unsigned g = grid_for(nc);
-    k_update<<<g, kThreads, sizeof(double2) * nvec, st>>>(V, nvec, nc, r, vcur, s.alpha + i + 1,
+    (void)launch_pdl(k_update, g, kThreads, sizeof(double2) * nvec, st, V, nvec, nc, r, vcur, s.alpha + i + 1,
                                                          s.coef, s.partial, s.done);
     return cudaGetLastError();
 }
@@ -408,7 +421,7 @@ cudaError_t launch_lanczos_reorth(const double2 *V, int nvec, double2 *r, int64_
 cudaError_t launch_lanczos_no_reorth(const double2 *vcur, double2 *r, int64_t nc, int i, LanczosState s,
                                      cudaStream_t st)
 {
-    k_update<<<grid_for(nc), kThreads, 0, st>>>(nullptr, 0, nc, r, vcur, s.alpha + i + 1, nullptr, s.partial,
+    (void)launch_pdl(k_update, grid_for(nc), kThreads, 0, st, nullptr, 0, nc, r, vcur, s.alpha + i + 1, nullptr, s.partial,
                                                 s.done);
     return cudaGetLastError();
 }
@@ -416,14 +429,14 @@ cudaError_t launch_lanczos_no_reorth(const double2 *vcur, double2 *r, int64_t nc
 cudaError_t launch_lanczos_axpy(const double2 *vprev, double2 *r, int64_t nc, int i, LanczosState s,
                                cudaStream_t st)
 {
-    k_axpy<<<grid_for(nc), kThreads, 0, st>>>(vprev, r, nc, s.beta + i, s.done);
+    (void)launch_pdl(k_axpy, grid_for(nc), kThreads, 0, st, vprev, r, nc, s.beta + i, s.done);
     return cudaGetLastError();
 }
 
 cudaError_t launch_axpy_real(double2 *acc, const double2 *v, int64_t nc, const double *z, int first,
                              cudaStream_t st)
 {
-    k_axpy_real<<<grid_for(nc), kThreads, 0, st>>>(acc, v, nc, z, first, nullptr);
+    (void)launch_pdl(k_axpy_real, grid_for(nc), kThreads, 0, st, acc, v, nc, z, first, nullptr);
     return cudaGetLastError();
 }
 
@@ -434,7 +447,7 @@ size_t shard_scratch_elems(int64_t n, int lm) { return lanczos_partial_elems(n, 
 cudaError_t launch_shard_scale(int64_t n, const double2 *r, double2 *vnext, const double *beta_i, const int *done,
                                cudaStream_t st)
 {
-    k_scale<<<grid_for(n), kThreads, 0, st>>>(r, vnext, n, beta_i, done);
+    (void)launch_pdl(k_scale, grid_for(n), kThreads, 0, st, r, vnext, n, beta_i, done);
     return cudaGetLastError();
 }
 
@@ -444,10 +457,10 @@ cudaError_t launch_shard_axpy_dot(int64_t n, const double2 *vprev, const double2
 {
     const unsigned g = grid_for(n);
     if (vprev)
-        k_axpy_dot<<<g, kThreads, 0, st>>>(vprev, vcur, r, n, beta_i, scratch, done);
+        (void)launch_pdl(k_axpy_dot, g, kThreads, 0, st, vprev, vcur, r, n, beta_i, scratch, done);
     else
-        k_dot_partial<<<g, kThreads, 0, st>>>(vcur, r, n, scratch, done);
-    k_sum_partials<<<1, kThreads, 0, st>>>(scratch, g, dot, done);
+        (void)launch_pdl(k_dot_partial, g, kThreads, 0, st, vcur, r, n, scratch, done);
+    (void)launch_pdl(k_sum_partials, 1, kThreads, 0, st, scratch, g, dot, done);
     return cudaGetLastError();
 }
 
@@ -456,8 +469,8 @@ cudaError_t launch_shard_multidot(int64_t n, const double2 *V, int nvec, const d
                                   cudaStream_t st)
 {
     const unsigned nblk = (unsigned)((n + kSlice - 1) / kSlice);
-    k_multidot<<<nblk ? nblk : 1, kThreads, 0, st>>>(V, nvec, n, r, vcur, alpha, scratch, done);
-    k_multidot_finish<<<(nvec + 7) / 8, kThreads, 0, st>>>(scratch, nblk, nvec, coef, done);
+    (void)launch_pdl(k_multidot, nblk ? nblk : 1, kThreads, 0, st, V, nvec, n, r, vcur, alpha, scratch, done);
+    (void)launch_pdl(k_multidot_finish, (nvec + 7) / 8, kThreads, 0, st, scratch, nblk, nvec, coef, done);
     return cudaGetLastError();
 }
 
@@ -466,23 +479,23 @@ cudaError_t launch_shard_update(int64_t n, const double2 *V, int nvec, double2 *
                                 const int *done, cudaStream_t st)
 {
     const unsigned g = grid_for(n);
-    k_update<<<g, kThreads, sizeof(double2) * (nvec > 0 ? nvec : 0), st>>>(V, nvec, n, r, vcur, alpha, coef,
+    (void)launch_pdl(k_update, g, kThreads, sizeof(double2) * (nvec > 0 ? nvec : 0), st, V, nvec, n, r, vcur, alpha, coef,
                                                                         scratch, done);
-    k_sum_partials_re<<<1, kThreads, 0, st>>>(scratch, g, norm2, done);
+    (void)launch_pdl(k_sum_partials_re, 1, kThreads, 0, st, scratch, g, norm2, done);
     return cudaGetLastError();
 }
 
 cudaError_t launch_shard_beta(int i, double tol, const double *norm2, double *beta, double *maxbeta, int *done,
                               int *iters, cudaStream_t st)
 {
-    k_beta_total<<<1, 32, 0, st>>>(norm2, i, tol, beta, maxbeta, done, iters);
+    (void)launch_pdl(k_beta_total, 1, 32, 0, st, norm2, i, tol, beta, maxbeta, done, iters);
     return cudaGetLastError();
 }
 
 cudaError_t launch_combine(const double2 *V, int nvec, int64_t nc, const double *z,
                            double2 *out, cudaStream_t st)
 {
-    k_combine<<<grid_for(nc), kThreads, sizeof(double) * nvec, st>>>(V, nvec, nc, z, out);
+    (void)launch_pdl(k_combine, grid_for(nc), kThreads, sizeof(double) * nvec, st, V, nvec, nc, z, out);
     return cudaGetLastError();
 }
 
