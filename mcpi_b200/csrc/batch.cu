@@ -6,8 +6,9 @@
 // member keeps the reference's recurrence (full classical Gram-Schmidt
 // reorthogonalisation, breakdown at beta_i / max beta < 1e-15) but each
 // stage is one launch over all members:
-//   * H.psi: per orbital count M one launch of the direct kernel (M <= 9,
-//     no intermediate) or one annihilation + one creation launch through the
+//   * H.psi: per orbital count M the contact form's two launches (M >= 10,
+//     contact interactions), one launch of the direct kernel (M <= 11, no
+//     intermediate) or one annihilation + one creation launch through the
 //     members' E (hpsi.cu, k_batch_*), blocks assigned from (member, block)
 //     work tables;
 //   * vector stages: blocks assigned from (member, 2048-row tile) work tables,
@@ -347,8 +348,19 @@ struct mcpi_batch_s {
             std::vector<unsigned char> vals;   // filled when the solve is captured
         };
         std::vector<Chunk> chunks;
+        // the contact form: members in pairs of launches of up to
+        // batch_contact_members(M)
+        struct Pair {
+            int2 *w1, *w2;   // (slot, block) work tables of configurations / rows
+            int n1, n2;
+            std::vector<int> members;
+            std::vector<unsigned char> vals;   // filled when the solve is captured
+        };
+        std::vector<Pair> pairs;
+        size_t sm0;        // shared memory of its first half
     };
     std::vector<char> mreal;   // member's block values are real
+    bool has_S = false;        // the arena has room for the contact form's S
     std::vector<Group> groups;
     // batched H.psi schedule (the autotuner's second dimension): bit 0 = the
     // M groups run as concurrent graph branches (else one after another),
@@ -408,20 +420,36 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
         const int ntiles = (int)((nc + mcpi::kTileMin - 1) / mcpi::kTileMin);   // room for any tile
         b->lz[m].nc = nc;
         b->lz[m].ntiles = ntiles;
-        off_V[m] = tot;
-        tot += mcpi::up256(sizeof(double2) * (size_t)lm * nc);
-        off_r[m] = tot;
-        tot += mcpi::up256(sizeof(double2) * nc);
-        off_E[m] = tot;
-        if (M[m] > mcpi::kBatchDirectMaxM)   // the two-kernel form's intermediate
-            tot += mcpi::up256(sizeof(double2) * (size_t)s->P * s->nc2);
-        off_S[m] = tot;
-        tot += mcpi::up256(sizeof(double2) * nc);
-        off_st[m] = tot;
-        tot += mcpi::up256(sizeof(double2) * (2 * (size_t)lm + (size_t)(lm + 1) * ntiles) +
-                           sizeof(double) * (lm + 1) + 2 * sizeof(int));
     }
-    if (cudaMalloc(&b->arena, tot) != cudaSuccess)
+    // the arena, with the contact form's intermediate for members that the
+    // direct form covers too as long as there is memory for it
+    for (int with_S = 1; with_S >= 0 && !b->arena; --with_S) {
+        tot = 0;
+        for (int m = 0; m < count; ++m) {
+            const mcpi_space_s *s = b->spaces[m];
+            const int64_t nc = s->nc;
+            off_V[m] = tot;
+            tot += mcpi::up256(sizeof(double2) * (size_t)lm * nc);
+            off_r[m] = tot;
+            tot += mcpi::up256(sizeof(double2) * nc);
+            off_E[m] = tot;
+            if (M[m] > mcpi::kBatchDirectMaxM)   // the two-kernel form's intermediate (the contact form's fits in it)
+                tot += mcpi::up256(sizeof(double2) * (size_t)s->P * s->nc2);
+            else if (with_S && M[m] >= mcpi::kBatchContactMinM)
+                tot += mcpi::up256(sizeof(double2) * (size_t)(2 * M[m] - 1) * s->nc2);
+            off_S[m] = tot;
+            tot += mcpi::up256(sizeof(double2) * nc);
+            off_st[m] = tot;
+            tot += mcpi::up256(sizeof(double2) * (2 * (size_t)lm + (size_t)(lm + 1) * b->lz[m].ntiles) +
+                               sizeof(double) * (lm + 1) + 2 * sizeof(int));
+        }
+        if (cudaMalloc(&b->arena, tot) != cudaSuccess) {
+            (void)cudaGetLastError();
+            b->arena = nullptr;
+        }
+        b->has_S = with_S != 0;
+    }
+    if (!b->arena)
         return cleanup(MCPI_ERR_NOMEM, "arena allocation failed (" + std::to_string(tot) + " bytes)");
     b->arena_bytes = tot;
     b->start.resize(count);
@@ -447,7 +475,9 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
         bm.nh = 0;
         bm.hdiag = nullptr;
         bm.lvec = z.V;
-        bm.E = M[m] > mcpi::kBatchDirectMaxM ? reinterpret_cast<double2 *>(b->arena + off_E[m]) : nullptr;
+        bm.E = M[m] > mcpi::kBatchDirectMaxM || (b->has_S && M[m] >= mcpi::kBatchContactMinM)
+                   ? reinterpret_cast<double2 *>(b->arena + off_E[m])
+                   : nullptr;
         bm.r = z.r;
         bm.done = z.done;
         bm.occ = bm.occ2 = nullptr;
@@ -506,6 +536,29 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
             cwi[g].push_back(ai);
         }
     }
+    // pairs of launches of the contact groups: (slot, block) tables
+    std::vector<std::vector<std::vector<int>>> pmem(Ms.size());
+    std::vector<std::vector<std::vector<int2>>> pw1(Ms.size()), pw2(Ms.size());
+    for (size_t g = 0; g < Ms.size(); ++g) {
+        if (Ms[g] < mcpi::kBatchContactMinM || !(b->has_S || Ms[g] > mcpi::kBatchDirectMaxM)) continue;
+        const int cap = mcpi::batch_contact_members(Ms[g]);
+        for (int m = 0; m < count; ++m) {
+            if (M[m] != Ms[g]) continue;
+            if (pmem[g].empty() || (int)pmem[g].back().size() == cap) pmem[g].emplace_back();
+            pmem[g].back().push_back(m);
+        }
+        for (const auto &mm : pmem[g]) {
+            std::vector<int2> a1, a2;
+            for (size_t sl = 0; sl < mm.size(); ++sl) {
+                const mcpi_space_s *s = b->spaces[mm[sl]];
+                for (int64_t k = 0; k * rpb1 < s->nc2; ++k) a1.push_back(make_int2((int)sl, (int)k));
+                // from the top rows down: their S entries were written last
+                for (int64_t k = (s->nc + rpb2 - 1) / rpb2 - 1; k >= 0; --k) a2.push_back(make_int2((int)sl, (int)k));
+            }
+            pw1[g].push_back(a1);
+            pw2[g].push_back(a2);
+        }
+    }
     size_t mbytes = mcpi::up256(sizeof(BatchLz) * count) + mcpi::up256(sizeof(BatchMember) * count) +
                     mcpi::up256(sizeof(int2) * vwork.size()) + mcpi::up256(sizeof(double) * count) +
                     mcpi::up256(sizeof(int) * count);
@@ -513,6 +566,8 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
         mbytes += 2 * (mcpi::up256(sizeof(int2) * w1[g].size()) + mcpi::up256(sizeof(int2) * w2[g].size()));
         for (size_t c = 0; c < cw[g].size(); ++c)
             mbytes += mcpi::up256(sizeof(int2) * cw[g][c].size()) + mcpi::up256(sizeof(int2) * cwi[g][c].size());
+        for (size_t c = 0; c < pw1[g].size(); ++c)
+            mbytes += mcpi::up256(sizeof(int2) * pw1[g][c].size()) + mcpi::up256(sizeof(int2) * pw2[g][c].size());
     }
     if (cudaMalloc(&b->meta, mbytes) != cudaSuccess) return cleanup(MCPI_ERR_NOMEM, "metadata allocation failed");
     char *p = b->meta;
@@ -572,7 +627,21 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
                 e = cudaMemcpy(C.wi, cwi[g][c].data(), sizeof(int2) * cwi[g][c].size(), cudaMemcpyHostToDevice);
             G.chunks.push_back(std::move(C));
         }
-        b->groups.push_back(G);
+        G.sm0 = mcpi::batch_smem(Ms[g], maxN, 0, 1);
+        for (size_t c = 0; c < pw1[g].size() && e == cudaSuccess; ++c) {
+            mcpi_batch_s::Group::Pair C;
+            C.w1 = reinterpret_cast<int2 *>(take(sizeof(int2) * pw1[g][c].size()));
+            C.w2 = reinterpret_cast<int2 *>(take(sizeof(int2) * pw2[g][c].size()));
+            C.n1 = (int)pw1[g][c].size();
+            C.n2 = (int)pw2[g][c].size();
+            C.members = pmem[g][c];
+            C.vals.assign(mcpi::batch_contact_bytes(Ms[g]), 0);
+            e = cudaMemcpy(C.w1, pw1[g][c].data(), sizeof(int2) * pw1[g][c].size(), cudaMemcpyHostToDevice);
+            if (e == cudaSuccess)
+                e = cudaMemcpy(C.w2, pw2[g][c].data(), sizeof(int2) * pw2[g][c].size(), cudaMemcpyHostToDevice);
+            G.pairs.push_back(std::move(C));
+        }
+        b->groups.push_back(std::move(G));
     }
     // side streams and events for the concurrent H.psi schedule
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
@@ -608,9 +677,9 @@ int mcpi_batch_set_integrals(mcpi_batch b, int member, const double *h_Ho, const
     bool real = true;
     for (const double2 &h : s->fwd.hblk_h) real = real && h.y == 0.0;
     b->mreal[member] = real;
-    if (b->exec)   // the real-valued direct form carries the values in the graph: capture again
+    if (b->exec)   // the real-valued direct and the contact form carry the values in the graph: capture again
         for (const auto &G : b->groups)
-            if (G.M == s->M && G.form == mcpi::kBatchDirectReal && b->exec) {
+            if (G.M == s->M && (G.form == mcpi::kBatchDirectReal || G.form == mcpi::kBatchContact) && b->exec) {
                 cudaStreamSynchronize(b->stream);
                 cudaGraphExecDestroy(b->exec);
                 cudaGraphDestroy(b->graph);
@@ -676,7 +745,13 @@ static cudaError_t enqueue_hpsi(mcpi_batch b, int vec, int sched)
     for (size_t g = 0; g < b->groups.size() && e == cudaSuccess; ++g) {
         const auto &G = b->groups[g];
         cudaStream_t s = branches && g > 0 ? b->side[g - 1] : st;
-        if (G.form == mcpi::kBatchDirectReal)
+        if (G.form == mcpi::kBatchContact)
+            for (size_t c = 0; c < G.pairs.size() && e == cudaSuccess; ++c) {
+                const auto &C = G.pairs[c];
+                e = mcpi::launch_batch_contact(G.M, b->d_mem, C.w1, C.n1, C.w2, C.n2, G.sm0, G.sm2, vec, C.vals.data(),
+                                               s);
+            }
+        else if (G.form == mcpi::kBatchDirectReal)
             for (size_t c = 0; c < G.chunks.size() && e == cudaSuccess; ++c)
                 e = mcpi::launch_batch_direct_vals(G.M, b->d_mem, inter ? G.chunks[c].wi : G.chunks[c].w,
                                                    G.chunks[c].n, G.sm3, vec, G.chunks[c].vals.data(), s);
@@ -870,7 +945,18 @@ int mcpi_batch_run(mcpi_batch b, double *h_E0, int *h_iters)
             bool real = true;
             for (int m = 0; m < b->count; ++m)
                 if (b->spaces[m]->M == G.M) real = real && b->mreal[m];
-            G.form = !G.direct ? mcpi::kBatchTwo : real ? mcpi::kBatchDirectReal : mcpi::kBatchDirectComplex;
+            bool contact = !G.pairs.empty();
+            for (int m = 0; m < b->count; ++m)
+                if (b->spaces[m]->M == G.M) contact = contact && !b->spaces[m]->fwd.contact.empty();
+            G.form = contact    ? mcpi::kBatchContact
+                     : !G.direct ? mcpi::kBatchTwo
+                     : real      ? mcpi::kBatchDirectReal
+                                 : mcpi::kBatchDirectComplex;
+            if (contact)
+                for (auto &C : G.pairs)
+                    for (size_t sl = 0; sl < C.members.size(); ++sl)
+                        mcpi::batch_fill_contact(G.M, C.vals.data(), (int)sl, C.members[sl],
+                                                 b->spaces[C.members[sl]]->fwd.contact.data());
             if (G.form == mcpi::kBatchDirectReal)
                 for (auto &C : G.chunks)
                     for (size_t sl = 0; sl < C.members.size(); ++sl)

@@ -1227,11 +1227,11 @@ struct ContactVals {
     double u[P], w[P];   // in pair_index order
 };
 
-template <int M>
-__global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb,
-                                                     const __grid_constant__ ContactVals<M> cv,
-                                                     const double2 *__restrict__ psi, double2 *__restrict__ S,
-                                                     uint32_t m0, uint32_t m1)
+// S_K(m) of configurations [m0 + block * kT2, ..) below m1; w(p): factor of pair p.
+template <int M, class WV>
+__device__ __forceinline__ void contact_sum_body(const Space &sp, const SpaceTables &tb, const WV &w,
+                                                 const double2 *__restrict__ psi, double2 *__restrict__ S,
+                                                 uint32_t block, uint32_t m0, uint32_t m1)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *sq = reinterpret_cast<double *>(smem_raw);            // wstride
@@ -1239,7 +1239,7 @@ __global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb
     load_tables(sp, tb, W, sq);
     pdl_wait();
     __syncthreads();
-    const uint32_t m = m0 + blockIdx.x * kT2 + threadIdx.x;
+    const uint32_t m = m0 + block * kT2 + threadIdx.x;
     if (m >= m1) return;
     const int ws = sp.wstride;
     int u[M], Q[M];
@@ -1273,7 +1273,7 @@ __global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb
         for (int c = 0; c < NB; ++c)
             if (c < n) {
                 const int q = qlo + c, l = K - q;
-                const double f = cv.w[pair_index(q, l, M)] * (fa[q] * ((q == l) ? sq[u[q] + 2] : fa[l]));
+                const double f = w(pair_index(q, l, M)) * (fa[q] * ((q == l) ? sq[u[q] + 2] : fa[l]));
                 s.x = fma(f, x[c].x, s.x);
                 s.y = fma(f, x[c].y, s.y);
             }
@@ -1282,12 +1282,21 @@ __global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb
 }
 
 template <int M>
-__global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables tb,
-                                                        const __grid_constant__ ContactVals<M> cv,
-                                                        const double2 *__restrict__ hdiag,
-                                                        const double2 *__restrict__ psi,
-                                                        const double2 *__restrict__ S, double2 *__restrict__ out,
-                                                        uint32_t row0, uint32_t row1)
+__global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb,
+                                                     const __grid_constant__ ContactVals<M> cv,
+                                                     const double2 *__restrict__ psi, double2 *__restrict__ S,
+                                                     uint32_t m0, uint32_t m1)
+{
+    contact_sum_body<M>(sp, tb, [&](int p) -> double { return cv.w[p]; }, psi, S, blockIdx.x, m0, m1);
+}
+
+// Rows [row0 + block * kTC, ..) below row1 into out[i - row0]; u(p): factor of pair p.
+template <int M, class UV>
+__device__ __forceinline__ void contact_create_body(const Space &sp, const SpaceTables &tb, const UV &u,
+                                                    const double2 *__restrict__ hdiag,
+                                                    const double2 *__restrict__ psi,
+                                                    const double2 *__restrict__ S, double2 *__restrict__ out,
+                                                    uint32_t block, uint32_t row0, uint32_t row1)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *r1 = reinterpret_cast<double *>(smem_raw);             // M x kTC
@@ -1301,8 +1310,7 @@ __global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables
     if (threadIdx.x < M) hd[threadIdx.x] = hdiag[threadIdx.x];
     pdl_wait();
     __syncthreads();
-    // from the top rows down: their S entries were written last, some are still in L2
-    const uint32_t i = row0 + (gridDim.x - 1 - blockIdx.x) * kTC + threadIdx.x;
+    const uint32_t i = row0 + block * kTC + threadIdx.x;
     if (i >= row1) return;
     const int t = threadIdx.x, ws = sp.wstride;
     double2 acc;
@@ -1349,7 +1357,7 @@ __global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables
                 const int s = k + rem;
                 const double c = r1[k * kTC + t] * ((s == k) ? sq[vb[k * kTC + t]] : r1[s * kTC + t]);
                 const uint32_t mm = Xr[k * kTC + t] - Yr[s * kTC + t];
-                cc[j] = c * cv.u[p];
+                cc[j] = c * u(p);
                 ee[j] = c == 0.0 ? make_double2(0.0, 0.0) : __ldg(S + (size_t)(k + s) * stride + mm);
             }
         }
@@ -1361,6 +1369,19 @@ __global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables
             }
     }
     out[i - row0] = acc;
+}
+
+template <int M>
+__global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables tb,
+                                                        const __grid_constant__ ContactVals<M> cv,
+                                                        const double2 *__restrict__ hdiag,
+                                                        const double2 *__restrict__ psi,
+                                                        const double2 *__restrict__ S, double2 *__restrict__ out,
+                                                        uint32_t row0, uint32_t row1)
+{
+    // from the top rows down: their S entries were written last, some are still in L2
+    contact_create_body<M>(sp, tb, [&](int p) -> double { return cv.u[p]; }, hdiag, psi, S, out,
+                           gridDim.x - 1 - blockIdx.x, row0, row1);
 }
 
 template <int M>
@@ -1769,6 +1790,44 @@ __global__ void __launch_bounds__(kTC, 3) k_batch_direct_p(const BatchMember *__
                                  b.lvec + (size_t)vec * b.sp.nc, b.r + i, i);
 }
 
+// The contact form for a batch: the members' factors as a kernel parameter (at
+// most 30 KB), read through the constant bank; two launches per chunk of members.
+template <int M>
+struct BatchContact {
+    static constexpr int P = M * (M + 1) / 2;
+    static constexpr int CAP = (30 * 1024) / (16 * P + 4) < 64 ? (30 * 1024) / (16 * P + 4) : 64;
+    double u[CAP][P], w[CAP][P];
+    int member[CAP];
+};
+
+template <int M>
+__global__ void __launch_bounds__(kT2, 4) k_batch_contact_sum(const BatchMember *__restrict__ mem,
+                                                           const int2 *__restrict__ work, int vec,
+                                                           const __grid_constant__ BatchContact<M> bc)
+{
+    const int2 wk = work[blockIdx.x];   // (slot in bc, block of the member's configurations)
+    const int slot = wk.x;
+    const BatchMember &b = mem[bc.member[slot]];
+    if (*b.done) return;
+    contact_sum_body<M>(b.sp, SpaceTables{b.W, b.sq, b.occ, b.occ_bits, b.occ2},
+                        [&](int p) -> double { return bc.w[slot][p]; }, b.lvec + (size_t)vec * b.sp.nc, b.E,
+                        (uint32_t)wk.y, 0u, b.sp.nc2);
+}
+
+template <int M>
+__global__ void __launch_bounds__(kTC, 4) k_batch_contact_create(const BatchMember *__restrict__ mem,
+                                                              const int2 *__restrict__ work, int vec,
+                                                              const __grid_constant__ BatchContact<M> bc)
+{
+    const int2 wk = work[blockIdx.x];   // (slot in bc, block of the member's rows)
+    const int slot = wk.x;
+    const BatchMember &b = mem[bc.member[slot]];
+    if (*b.done) return;
+    contact_create_body<M>(b.sp, SpaceTables{b.W, b.sq, b.occ, b.occ_bits, b.occ2},
+                           [&](int p) -> double { return bc.u[slot][p]; }, b.hdiag, b.lvec + (size_t)vec * b.sp.nc,
+                           b.E, b.r, (uint32_t)wk.y, 0u, b.sp.nc);
+}
+
 template <int M>
 cudaError_t batch_prepare_m(size_t smem1, size_t smem2, size_t smem3)
 {
@@ -1782,6 +1841,8 @@ cudaError_t batch_prepare_m(size_t smem1, size_t smem2, size_t smem3)
         e = cudaFuncSetAttribute(k_batch_direct<M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_batch_direct_p<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_batch_contact_create<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
     return e;
 }
 
@@ -2007,6 +2068,82 @@ cudaError_t launch_batch_direct_vals(int M, const BatchMember *mem, const int2 *
     case m:                                                                                              \
         k_batch_direct_p<m><<<n, kTC, smem, st>>>(mem, work, vec, *static_cast<const BatchVals<m> *>(vals)); \
         return cudaGetLastError();
+        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
+        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
+        MCPI_CASE(15) MCPI_CASE(16)
+#undef MCPI_CASE
+    default: return cudaErrorInvalidValue;
+    }
+}
+
+int batch_contact_members(int M)
+{
+    switch (M) {
+#define MCPI_CASE(m) \
+    case m: return BatchContact<m>::CAP;
+        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
+        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
+        MCPI_CASE(15) MCPI_CASE(16)
+#undef MCPI_CASE
+    default: return 0;
+    }
+}
+
+size_t batch_contact_bytes(int M)
+{
+    switch (M) {
+#define MCPI_CASE(m) \
+    case m: return sizeof(BatchContact<m>);
+        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
+        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
+        MCPI_CASE(15) MCPI_CASE(16)
+#undef MCPI_CASE
+    default: return 0;
+    }
+}
+
+namespace {
+template <int M>
+void fill_contact_m(void *vals, int slot, int member, const double *uw)
+{
+    auto *bc = static_cast<BatchContact<M> *>(vals);
+    bc->member[slot] = member;
+    for (int x = 0; x < BatchContact<M>::P; ++x) {
+        bc->u[slot][x] = uw[x];
+        bc->w[slot][x] = uw[BatchContact<M>::P + x];
+    }
+}
+
+template <int M>
+cudaError_t launch_contact_m(const BatchMember *mem, const int2 *work1, int n1, const int2 *work2, int n2,
+                             size_t smem1, size_t smem2, int vec, const void *vals, cudaStream_t st)
+{
+    const auto &bc = *static_cast<const BatchContact<M> *>(vals);
+    if (n1) k_batch_contact_sum<M><<<n1, kT2, smem1, st>>>(mem, work1, vec, bc);
+    if (n2) k_batch_contact_create<M><<<n2, kTC, smem2, st>>>(mem, work2, vec, bc);
+    return cudaGetLastError();
+}
+}  // namespace
+
+void batch_fill_contact(int M, void *vals, int slot, int member, const double *uw)
+{
+    switch (M) {
+#define MCPI_CASE(m) \
+    case m: fill_contact_m<m>(vals, slot, member, uw); break;
+        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
+        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
+        MCPI_CASE(15) MCPI_CASE(16)
+#undef MCPI_CASE
+    default: break;
+    }
+}
+
+cudaError_t launch_batch_contact(int M, const BatchMember *mem, const int2 *work1, int n1, const int2 *work2, int n2,
+                                 size_t smem1, size_t smem2, int vec, const void *vals, cudaStream_t st)
+{
+    switch (M) {
+#define MCPI_CASE(m) \
+    case m: return launch_contact_m<m>(mem, work1, n1, work2, n2, smem1, smem2, vec, vals, st);
         MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
         MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
         MCPI_CASE(15) MCPI_CASE(16)

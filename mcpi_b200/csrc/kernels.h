@@ -181,7 +181,7 @@ struct BatchMember {
     int nh;
     const double2 *hdiag;    // Ho[k][k]
     const double2 *lvec;     // Krylov basis, vector k at lvec + k * nc
-    double2 *E;              // P x nc2 intermediate
+    double2 *E;              // P x nc2 intermediate ((2M-1) x nc2 in the contact form)
     double2 *r;              // H.psi output (the Lanczos residual)
     const int *done;         // this member's breakdown flag
     const uint64_t *occ;     // packed occupations of the N and N-2 spaces (or null: decode)
@@ -194,7 +194,7 @@ struct BatchMember {
 // Krylov vector each member applies H to. form: the two pair kernels
 // (members need E), or the direct kernel over work2's row blocks with smem2
 // = batch_smem(M, N, nh, 3) (real or complex block values).
-enum { kBatchTwo = 0, kBatchDirectReal = 1, kBatchDirectComplex = 2 };
+enum { kBatchTwo = 0, kBatchDirectReal = 1, kBatchDirectComplex = 2, kBatchContact = 3 };
 // Orbital counts up to which a batch takes the direct form (the single-space
 // default's range).
 constexpr int kBatchDirectMaxM = 11;
@@ -211,6 +211,19 @@ size_t batch_vals_bytes(int M);
 void batch_fill_vals(int M, void *vals, int slot, int member, const double2 *hblk_host);
 cudaError_t launch_batch_direct_vals(int M, const BatchMember *mem, const int2 *work, int n, size_t smem, int vec,
                                      const void *vals, cudaStream_t st);
+// The contact form (every member's blocks are outer products; E holds S): up
+// to batch_contact_members(M) members per pair of launches, their factors u[P]
+// | w[P] in a host buffer of batch_contact_bytes(M) bytes; work lists (slot,
+// block) of configurations (work1, smem1 = batch_smem(M, N, 0, 1)) and rows
+// (work2, smem2 = batch_smem(.., 2)).
+int batch_contact_members(int M);
+size_t batch_contact_bytes(int M);
+void batch_fill_contact(int M, void *vals, int slot, int member, const double *uw);
+cudaError_t launch_batch_contact(int M, const BatchMember *mem, const int2 *work1, int n1, const int2 *work2, int n2,
+                                 size_t smem1, size_t smem2, int vec, const void *vals, cudaStream_t st);
+// Orbital counts from which a batch takes the contact form where it can (its
+// members share the launches, so their sizes do not matter as in contact_pays).
+constexpr int kBatchContactMinM = 10;
 // Sets the kernels' shared-memory limits (call outside stream capture).
 cudaError_t batch_prepare(int M, size_t smem1, size_t smem2, size_t smem3);
 // configurations per block of the batched kernels: stage 1 annihilation, 2 creation

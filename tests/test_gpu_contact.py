@@ -125,3 +125,47 @@ def test_capture_uses_the_direct_form():
     assert float(torch.linalg.vector_norm(out - ref) / torch.linalg.vector_norm(ref)) <= TOL
     del g
     sp.close()
+
+
+def test_batched_contact_groups_follow_their_integrals():
+    # groups of M = 10, 11, 12 take the contact form; one member with another
+    # interaction moves its group to the direct or two-kernel form at the next
+    # run, and back. E0 against single solves at the repository's 1e-10.
+    lm = 40
+    members = [(6, 10), (4, 10), (5, 11), (7, 11), (3, 12), (5, 12), (6, 7)]
+    i = np.arange(16)
+
+    def finite_range(M, g):
+        Ho, _ = mc.lieb_integrals(M, g)
+        l, q, s, k = np.meshgrid(i[:M], i[:M], i[:M], i[:M], indexing="ij")
+        v = lambda p: np.exp(-0.06 * p.astype(float) ** 2)
+        return Ho, np.where(k + s == q + l, 0.5 * g * (v(k - l) + v(k - q)), 0.0).reshape(-1).astype(np.complex128)
+
+    contact = [mc.lieb_integrals(M, 0.5 + 0.7 * x) for x, (N, M) in enumerate(members)]
+    other = [finite_range(M, 1.5) for N, M in members]
+    starts = [mc.random_problem(N, M, 60 + x)[0] for x, (N, M) in enumerate(members)]
+
+    def singles(ints):
+        out = []
+        for (N, M), (Ho, Hint), C in zip(members, ints, starts):
+            sp = mc.FockSpace(N, M)
+            sp.set_option(mc.OPT_DIRECT_HPSI, 1)
+            sp.set_integrals(Ho, Hint)
+            out.append(sp.ground(C, lm)[0])
+            sp.close()
+        return np.array(out)
+
+    b = mc.Batch(members, lm)
+    for x in range(len(members)):
+        b.set_integrals(x, *contact[x])
+        b.set_start(x, starts[x])
+    mixed = list(contact)
+    for changed in ([], [1, 3, 5], [1, 3, 5]):
+        for x in changed:
+            mixed[x] = other[x] if mixed[x] is contact[x] else contact[x]
+            b.set_integrals(x, *mixed[x])
+        E, it = b.run()
+        ref = singles(mixed)
+        assert (it == lm).all()
+        assert np.abs(E - ref).max() <= 1e-10 * max(1.0, np.abs(ref).max())
+    b.close()
