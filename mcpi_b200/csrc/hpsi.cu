@@ -1220,6 +1220,15 @@ cudaError_t direct_apply_m(const Space &sp, const SpaceTables &tb, const PairOp 
 // total momentum instead of one per creation pair:
 //     S_K(m) = sum_{b in block K} w_b c_b(m) psi[m + b],
 //     (H2 psi)(v) = sum_{a in v} u_a c_a(v) S_{K(a)}(v - a).
+// Kernel 1 gathers P values per (N-2)-configuration and stores 2M-1 sums;
+// kernel 2 gathers one sum per occupied pair of a row. Against the 60 % of
+// predicated-off products of the direct form, that is 90 M gathers of 16 bytes
+// at N=16, M=10 instead of 114 M, and a third of the instructions. Both are
+// bound by the L1 data pipe (72 % and 66 % of peak: consecutive rows gather in
+// short unaligned runs, 8 wavefronts per full request), kernel 2 by issue too
+// (61 %); DRAM carries 0.6 GB. 78 + 133 us at N=16, M=10. Blocks per SM: kernel 1
+// three (80 registers; four spill: 35 against 31 us at N=12, M=11), kernel 2
+// four up to ten orbitals and three above (N=9, M=13 35 -> 32 us).
 // ---------------------------------------------------------------------------
 template <int M>
 struct ContactVals {
@@ -1282,7 +1291,7 @@ __device__ __forceinline__ void contact_sum_body(const Space &sp, const SpaceTab
 }
 
 template <int M>
-__global__ void __launch_bounds__(kT2, 4) k_contact_sum(Space sp, SpaceTables tb,
+__global__ void __launch_bounds__(kT2, 3) k_contact_sum(Space sp, SpaceTables tb,
                                                      const __grid_constant__ ContactVals<M> cv,
                                                      const double2 *__restrict__ psi, double2 *__restrict__ S,
                                                      uint32_t m0, uint32_t m1)
@@ -1372,7 +1381,7 @@ __device__ __forceinline__ void contact_create_body(const Space &sp, const Space
 }
 
 template <int M>
-__global__ void __launch_bounds__(kTC, 4) k_contact_create(Space sp, SpaceTables tb,
+__global__ void __launch_bounds__(kTC, M <= 10 ? 4 : 3) k_contact_create(Space sp, SpaceTables tb,
                                                         const __grid_constant__ ContactVals<M> cv,
                                                         const double2 *__restrict__ hdiag,
                                                         const double2 *__restrict__ psi,
@@ -1431,9 +1440,10 @@ bool contact_pays(const Space &sp)
 {
     if (!direct_covers(sp)) return true;   // stands in for the two pair kernels
     // against the direct form, measured in us (contact / direct) on rotating
-    // states: M=11 N=10 33 / 35, N=12 77 / 97, N=16 582 / 750; M=10 N=11 28 / 25,
-    // N=12 37 / 37, N=13 58 / 74, N=16 205 / 226, N=18 475 / 512, N=20 1154 / 1117
-    // (S then no longer has a useful share in L2); M=9 N=16 75 / 68, N=20 294 / 274
+    // states: M=11 N=10 33 / 35, N=12 69 / 95, N=16 582 / 750; M=10 N=11 28 / 25,
+    // N=12 37 / 37, N=13 58 / 74, N=16 204 / 225, N=18 475 / 512, N=20 1142 / 1118
+    // (its S, 1.4 GB, and the states then leave each other nothing in L2); M=9
+    // N=16 70 / 65, N=20 294 / 274
     return sp.M == 11 ? sp.nc >= 180000 : sp.M == 10 && sp.nc >= 290000 && sp.nc <= 6000000;
 }
 
@@ -1801,7 +1811,7 @@ struct BatchContact {
 };
 
 template <int M>
-__global__ void __launch_bounds__(kT2, 4) k_batch_contact_sum(const BatchMember *__restrict__ mem,
+__global__ void __launch_bounds__(kT2, 3) k_batch_contact_sum(const BatchMember *__restrict__ mem,
                                                            const int2 *__restrict__ work, int vec,
                                                            const __grid_constant__ BatchContact<M> bc)
 {
@@ -1815,7 +1825,7 @@ __global__ void __launch_bounds__(kT2, 4) k_batch_contact_sum(const BatchMember 
 }
 
 template <int M>
-__global__ void __launch_bounds__(kTC, 4) k_batch_contact_create(const BatchMember *__restrict__ mem,
+__global__ void __launch_bounds__(kTC, M <= 10 ? 4 : 3) k_batch_contact_create(const BatchMember *__restrict__ mem,
                                                               const int2 *__restrict__ work, int vec,
                                                               const __grid_constant__ BatchContact<M> bc)
 {
