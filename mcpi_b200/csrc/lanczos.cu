@@ -160,7 +160,9 @@ __global__ void __launch_bounds__(kThreads) k_multidot(const double2 *__restrict
     }
     __syncthreads();
     const int w = threadIdx.x / 32, lane = threadIdx.x % 32;
-    for (int j = w; j < nvec; j += kThreads / 32) {
+    // the vectors are split over the grid's y blocks (multidot_grid); which warp
+    // takes one does not change its sum
+    for (int j = w + blockIdx.y * (kThreads / 32); j < nvec; j += gridDim.y * (kThreads / 32)) {
         const double2 *vj = V + (size_t)j * n + r0;
         double2 acc = make_double2(0.0, 0.0);
 #pragma unroll 4
@@ -343,6 +345,18 @@ static unsigned grid_for(int64_t n)
     return (unsigned)(g < kParts ? (g > 0 ? g : 1) : kParts);
 }
 
+// Blocks of k_multidot: one per 1024-row slice, times as many as it takes for
+// the slices of a small vector to fill the chip (592 blocks: four per SM), at
+// most one warp per basis vector. Every y block stages its slice of x again, so
+// large vectors keep one. (100 steps, y = 1 / this: N=10, M=9
+// 5.42 / 3.48 ms, N=10, M=10 9.34 / 5.83 ms, N=12, M=10 16.1 / 14.0 ms.)
+static dim3 multidot_grid(unsigned nblk, int nvec)
+{
+    const unsigned most = (unsigned)(nvec + 7) / 8, want = nblk ? (unsigned)kParts / nblk : 1;
+    const unsigned y = want < most ? want : most;
+    return dim3(nblk ? nblk : 1, y ? y : 1);
+}
+
 int lanczos_parts(int64_t nc)
 {
     return (int)grid_for(nc);
@@ -409,7 +423,7 @@ cudaError_t launch_lanczos_reorth(const double2 *V, int nvec, double2 *r, int64_
 {
     const double2 *vcur = V + (size_t)(i + 1) * nc;
     const unsigned nblk = (unsigned)((nc + kSlice - 1) / kSlice);
-    (void)launch_pdl(k_multidot, nblk, kThreads, 0, st, V, nvec, nc, r, vcur, s.alpha + i + 1, s.partial, s.done);
+    (void)launch_pdl(k_multidot, multidot_grid(nblk, nvec), kThreads, 0, st, V, nvec, nc, r, vcur, s.alpha + i + 1, s.partial, s.done);
     (void)launch_pdl(k_multidot_finish, (nvec + 7) / 8, kThreads, 0, st, s.partial, nblk, nvec, s.coef, s.done);
     const unsigned g = grid_for(nc);
     (void)launch_pdl(k_update, g, kThreads, sizeof(double2) * nvec, st, V, nvec, nc, r, vcur, s.alpha + i + 1,
@@ -469,7 +483,7 @@ cudaError_t launch_shard_multidot(int64_t n, const double2 *V, int nvec, const d
                                   cudaStream_t st)
 {
     const unsigned nblk = (unsigned)((n + kSlice - 1) / kSlice);
-    (void)launch_pdl(k_multidot, nblk ? nblk : 1, kThreads, 0, st, V, nvec, n, r, vcur, alpha, scratch, done);
+    (void)launch_pdl(k_multidot, multidot_grid(nblk, nvec), kThreads, 0, st, V, nvec, n, r, vcur, alpha, scratch, done);
     (void)launch_pdl(k_multidot_finish, (nvec + 7) / 8, kThreads, 0, st, scratch, nblk, nvec, coef, done);
     return cudaGetLastError();
 }
