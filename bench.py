@@ -169,7 +169,7 @@ def measured_peak():
 
 def ncu_figure(key, kernel):
     """A per-kernel figure (`key kernel value` line) from the committed ncu summaries, or None."""
-    for name in ("hpsi_direct_lieb_n16_m10.md", "hpsi_lieb_n16_m10.md"):
+    for name in ("hpsi_contact_lieb_n16_m10.md", "hpsi_direct_lieb_n16_m10.md", "hpsi_lieb_n16_m10.md"):
         p = os.path.join(ROOT, "profiles", name)
         if not os.path.exists(p):
             continue
@@ -189,6 +189,12 @@ def hpsi_bytes(nc, nc2, P):
     reads psi once and writes the P x nc2 intermediate E; kernel 2 reads E and
     psi and writes out (16 B per complex)."""
     return {"pair_annihilate": 16 * nc + 16 * P * nc2, "pair_create": 16 * P * nc2 + 32 * nc}
+
+
+def contact_bytes(nc, nc2, M):
+    """Algorithmic HBM bytes per launch of the two kernels of the contact form:
+    the same with S, one row per total momentum (2M-1), in the place of E."""
+    return {"contact_sum": 16 * nc + 16 * (2 * M - 1) * nc2, "contact_create": 16 * (2 * M - 1) * nc2 + 32 * nc}
 
 
 def direct_bytes(nc):
@@ -659,19 +665,23 @@ def run_mcpi(args):
                              "issue_active_pct": ncu_figure("issue_active_pct", dom),
                              "source": "profiles/hpsi_direct_lieb_n16_m10.md"}}
     else:
-        names = ["pair_annihilate", "pair_create"]
-        times = {"pair_annihilate": k1, "pair_create": k2}
-        dom = max(names, key=lambda n: times[n])
-        byts = hpsi_bytes(nc, nc2, P)
+        # the contact form (the default for a contact interaction at this size)
+        times = {"contact_sum": k1, "contact_create": k2}
+        dom = max(times, key=lambda n: times[n])
+        byts = contact_bytes(nc, nc2, M)
         t_dom, b_dom, kernel_ms = times[dom], byts[dom], times
-        extra = {"irreducible_bytes": 32 * nc}
+        extra = {"irreducible_bytes": 32 * nc, "gathers_per_step": 2 * P * nc2,
+                 "binding": {"unit": "SM L1 data pipe (16-byte gathers in short unaligned runs), then issue",
+                             "l1_data_pipe_pct": ncu_figure("l1_data_pipe_pct", dom),
+                             "issue_active_pct": ncu_figure("issue_active_pct", dom),
+                             "source": "profiles/hpsi_contact_lieb_n16_m10.md"}}
     achieved = b_dom / (t_dom * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": peak_kind,
                 "traffic": ncu_traffic(dom), "algorithmic_bytes": b_dom, **extra, "kernel_ms": kernel_ms}
-    # the two pair kernels on the same states, for comparison (MCPI_OPT_DIRECT_HPSI = 0)
-    if k2 == 0.0:
-        sp.set_option(mc.OPT_DIRECT_HPSI, 0)
+    # the other forms on the same states, for comparison (MCPI_OPT_DIRECT_HPSI = 1, 0)
+    for key, opt in (("direct_form_ms", 1), ("two_kernel_form_ms", 0)):
+        sp.set_option(mc.OPT_DIRECT_HPSI, opt)
         for w in range(3):
             sp.apply_h(X[w % ROTATE], out)
         t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -680,8 +690,8 @@ def run_mcpi(args):
             sp.apply_h(X[k % ROTATE], out)
         t1.record()
         torch.cuda.synchronize()
-        roofline["two_kernel_form_ms"] = t0.elapsed_time(t1) / args.steps
-        sp.set_option(mc.OPT_DIRECT_HPSI, 2)
+        roofline[key] = t0.elapsed_time(t1) / args.steps
+    sp.set_option(mc.OPT_DIRECT_HPSI, 2)
 
     # ---- e2e through the C ABI with HOST buffers (mcpi_apply_h_host) ----
     # every step copies its state in from pinned host memory and its result
@@ -802,7 +812,7 @@ def run_profile(args):
     of the N=16, M=10 workload after a warm-up solve; 'density' = rho1, rho2
     and the transition rho2 of seeded N=16, M=10 states (--steps calls each
     after --warmup, CUDA events); 'hpsi' = H.psi of the N=16, M=10 workload
-    with the two pair kernels, the fused kernel and the direct kernel."""
+    with the two pair kernels, the fused kernel, the direct kernel and the contact form."""
     import torch
 
     import mcpi_b200 as mc
@@ -846,17 +856,17 @@ def run_profile(args):
             out[name + "_ms"] = a.elapsed_time(b) / args.steps
         sp.close()
     elif args.profile == "hpsi":
-        # H.psi of the N=16, M=10 workload in its three forms: the two pair
-        # kernels, the fused kernel (MCPI_OPT_FUSED_HPSI; lead 192) and the
-        # direct kernel (MCPI_OPT_DIRECT_HPSI), --steps calls each on rotating
+        # H.psi of the N=16, M=10 workload in its forms: the two pair
+        # kernels, the fused kernel (MCPI_OPT_FUSED_HPSI; lead 192), the direct
+        # kernel (MCPI_OPT_DIRECT_HPSI) and the contact form (default), --steps calls each on rotating
         # states after --warmup. The fused form agrees with the two kernels bit
-        # for bit; the direct form sums in another order (relative difference)
+        # for bit; the others sum in another order (relative difference)
         gen = torch.Generator(device="cuda:0")
         gen.manual_seed(1234)
         X = None
         out = {"section": "hpsi", "workload": f"Lieb-Liniger N={N_PART} M={M_ORB}"}
         ref = None
-        for name, fused, direct in (("two_kernels", 0, 0), ("fused", 1, 0), ("direct", 0, 1)):
+        for name, fused, direct in (("two_kernels", 0, 0), ("fused", 1, 0), ("direct", 0, 1), ("contact", 0, 2)):
             sp = mc.FockSpace(N_PART, M_ORB, device=0)
             sp.set_option(mc.OPT_DIRECT_HPSI, direct)
             sp.set_option(mc.OPT_FUSED_HPSI, fused)
@@ -881,7 +891,7 @@ def run_profile(args):
             elif name == "fused":
                 out["fused_bitwise_equal"] = bool(torch.equal(ref, z))
             else:
-                out["direct_rel_diff"] = float(torch.linalg.vector_norm(z - ref) / torch.linalg.vector_norm(ref))
+                out[name + "_rel_diff"] = float(torch.linalg.vector_norm(z - ref) / torch.linalg.vector_norm(ref))
             sp.close()
     else:
         sp = mc.FockSpace(N_PART, M_ORB, device=0)
