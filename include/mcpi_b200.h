@@ -103,7 +103,9 @@ MCPI_API int mcpi_space_sync(mcpi_space sp);
 /* MCPI_OPT_DIRECT_HPSI: apply momentum-block integrals row by row, gathering
  * every term straight from the state, with no P x NC(N-2,M) intermediate
  * (N < 64; whole vectors and row ranges alike).
- * 0 off, 1 on, 2 (default) on for M <= 11, where it is the faster form. */
+ * 0 off, 1 on, 2 (default) on for M <= 11, where it is the faster form, except
+ * that contact interactions (every momentum block an outer product u_a w_b)
+ * take two kernels over one sum per total momentum where those are faster. */
 #define MCPI_OPT_DIRECT_HPSI 11
 MCPI_API int mcpi_space_set_option(mcpi_space sp, int option, int value);
 MCPI_API int mcpi_space_dims(mcpi_space sp, int *N, int *M, int64_t *nc);
@@ -161,8 +163,9 @@ MCPI_API int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int
 /* mcpi_apply_h, timed: runs it reps times with CUDA events around each of its
  * two kernels on the space's stream (synchronising after every repetition) and
  * returns their mean durations in ms: h_ms[0] pair annihilation + pair-matrix
- * kernel, h_ms[1] pair creation kernel (where the call takes the direct or
- * the fused one-kernel form: h_ms[0] that kernel, h_ms[1] = 0). For
+ * kernel, h_ms[1] pair creation kernel (in the contact form: its two kernels;
+ * where the call takes the direct or the fused one-kernel form: h_ms[0] that
+ * kernel, h_ms[1] = 0). For
  * measurement, not for production. */
 MCPI_API int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, float *h_ms);
 /* out = H C without allocating anything. No counterpart in the reference.
