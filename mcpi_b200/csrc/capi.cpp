@@ -1302,10 +1302,11 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
     if (rc) return rc;
     rc = reserve(sp, sp->d_lzr, sp->lzr_cap, sizeof(double2) * nc);
     if (rc) return rc;
-    const bool small = small_lanczos(sp, lm);
-    if (small) {
-        rc = reserve(sp, sp->d_small, sp->small_cap, mcpi::small_lanczos_bytes(sp->sp, lm));
-        if (rc) return rc;
+    // the one-launch form where its lists fit the device too
+    bool small = small_lanczos(sp, lm);
+    if (small && reserve(sp, sp->d_small, sp->small_cap, mcpi::small_lanczos_bytes(sp->sp, lm)) != MCPI_OK) {
+        (void)cudaGetLastError();
+        small = false;
     }
     char *blk = (char *)sp->d_lzblk;
     double2 *r = (double2 *)sp->d_lzr;
