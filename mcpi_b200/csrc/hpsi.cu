@@ -37,6 +37,19 @@ constexpr int kT2 = 256;   // threads per block, kernel 2 (register form) and ke
 constexpr int kTC = 256;   // threads (= rows) per block, kernel 2 (shared-table form)
 constexpr int kCreateBatch = 8;   // E gathers issued together per thread, kernel 2 (shared-table form)
 
+// Where v_o - 1 of the row of thread t lies among the 16-bit values: two orbitals
+// to a 32-bit column word, so that its address shares the register of Xr and Yr.
+// (16 bits: up to about 2,000 particles sit in one orbital.)
+constexpr __host__ __device__ int vcol(int o, int t) { return (o / 2) * 2 * kTC + 2 * t + o % 2; }
+
+// Shared memory of a row block of kernel 2 without the space's tables: r1, Xr,
+// Yr and v - 1 per orbital and row, then hd.
+constexpr size_t create_smem(int M)
+{
+    return (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + sizeof(uint32_t) * ((M + 1) / 2) * kTC +
+           sizeof(double2) * M;
+}
+
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 {
     unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -847,7 +860,7 @@ __global__ void __launch_bounds__(kT2, 4) k_pair_create(Space sp, SpaceTables tb
 // Kernel 2, shared-table form (default): the per-row tables (Xr, Yr, sqrt v_k
 // and v_k - 1) live in shared-memory columns that only their thread touches,
 // so the pair loop needs few registers (no spills) and occupancy is set by
-// shared memory (17 bytes per orbital and row). Measured at N=16, M=10:
+// shared memory (18 bytes per orbital and row). Measured at N=16, M=10:
 // 0.183 ms with the E gathers issued in groups of 8 (0.198 ms consumed one by
 // one, 0.186 ms in groups of 16), against 0.238 ms with two double tables, 0.248 ms for the register
 // form, 0.216 ms keeping only occupation bytes (square roots looked up per
@@ -864,7 +877,7 @@ __device__ __forceinline__ void create_row(const Space &sp, const SpaceTables &t
                                            const double *sq, const double2 *hd,
                                            const double2 *__restrict__ psi, const double2 *E,
                                            double2 *__restrict__ out, uint32_t i, bool row, uint32_t row0,
-                                           double *r1, uint32_t *Xr, uint32_t *Yr, unsigned char *vb,
+                                           double *r1, uint32_t *Xr, uint32_t *Yr, uint16_t *vb,
                                            uint64_t pol)
 {
     const int t = threadIdx.x;
@@ -894,7 +907,7 @@ __device__ __forceinline__ void create_row(const Space &sp, const SpaceTables &t
             Xr[o * kTC + t] = base - (A0[o] - Am1[o]);
             Yr[o * kTC + t] = Am1[o] - Am2[o];
             r1[o * kTC + t] = row ? sq[v[o]] : 0.0;
-            vb[o * kTC + t] = (unsigned char)(v[o] >= 1 ? v[o] - 1 : 0);
+            vb[vcol(o, t)] = (uint16_t)(v[o] >= 1 ? v[o] - 1 : 0);
         }
     }
     const size_t stride = sp.nc2;
@@ -919,7 +932,7 @@ __device__ __forceinline__ void create_row(const Space &sp, const SpaceTables &t
                         k = kk + 1;
                     }
                 const int s = k + rem;
-                const double c = r1[k * kTC + t] * ((s == k) ? sq[vb[k * kTC + t]] : r1[s * kTC + t]);
+                const double c = r1[k * kTC + t] * ((s == k) ? sq[vb[vcol(k, t)]] : r1[s * kTC + t]);
                 const uint32_t mm = Xr[k * kTC + t] - Yr[s * kTC + t];
                 cc[j] = c;
                 // empty pairs (c = 0: their index is meaningless) load nothing
@@ -945,7 +958,7 @@ __device__ __forceinline__ void create_row(const Space &sp, const SpaceTables &t
 // Kernel 2, shared-table form (default): the per-row tables (Xr, Yr, sqrt v_k
 // and v_k - 1) live in shared-memory columns that only their thread touches,
 // so the pair loop needs few registers (no spills) and occupancy is set by
-// shared memory (17 bytes per orbital and row). Measured at N=16, M=10:
+// shared memory (18 bytes per orbital and row). Measured at N=16, M=10:
 // 0.183 ms with the E gathers issued in groups of 8 (0.198 ms consumed one by
 // one, 0.186 ms in groups of 16), against 0.238 ms with two double tables, 0.248 ms for the register
 // form, 0.216 ms keeping only occupation bytes (square roots looked up per
@@ -964,8 +977,8 @@ __device__ __forceinline__ void create_smem_body(const Space &sp, const SpaceTab
     double *r1 = reinterpret_cast<double *>(smem_raw);             // M x kTC
     uint32_t *Xr = reinterpret_cast<uint32_t *>(r1 + M * kTC);     // M x kTC
     uint32_t *Yr = Xr + M * kTC;                                   // M x kTC
-    unsigned char *vb = reinterpret_cast<unsigned char *>(Yr + M * kTC);   // M x kTC
-    double2 *hd = reinterpret_cast<double2 *>(vb + ((M * kTC + 15) & ~15)); // M
+    uint16_t *vb = reinterpret_cast<uint16_t *>(Yr + M * kTC);     // (M + 1) / 2 x 2 kTC (vcol)
+    double2 *hd = reinterpret_cast<double2 *>(vb + (M + 1) / 2 * 2 * kTC); // M
     double *sq = reinterpret_cast<double *>(hd + M);               // wstride
     uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);   // (M-1) x wstride
     load_tables(sp, tb, W, sq);
@@ -1311,8 +1324,8 @@ __device__ __forceinline__ void contact_create_body(const Space &sp, const Space
     double *r1 = reinterpret_cast<double *>(smem_raw);             // M x kTC
     uint32_t *Xr = reinterpret_cast<uint32_t *>(r1 + M * kTC);     // M x kTC
     uint32_t *Yr = Xr + M * kTC;                                   // M x kTC
-    unsigned char *vb = reinterpret_cast<unsigned char *>(Yr + M * kTC);   // M x kTC
-    double2 *hd = reinterpret_cast<double2 *>(vb + ((M * kTC + 15) & ~15)); // M
+    uint16_t *vb = reinterpret_cast<uint16_t *>(Yr + M * kTC);     // (M + 1) / 2 x 2 kTC (vcol)
+    double2 *hd = reinterpret_cast<double2 *>(vb + (M + 1) / 2 * 2 * kTC); // M
     double *sq = reinterpret_cast<double *>(hd + M);               // wstride
     uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);   // (M-1) x wstride
     load_tables(sp, tb, W, sq);
@@ -1343,7 +1356,7 @@ __device__ __forceinline__ void contact_create_body(const Space &sp, const Space
             Xr[o * kTC + t] = base - (A0[o] - Am1[o]);
             Yr[o * kTC + t] = Am1[o] - Am2[o];
             r1[o * kTC + t] = sq[v[o]];
-            vb[o * kTC + t] = (unsigned char)(v[o] >= 1 ? v[o] - 1 : 0);
+            vb[vcol(o, t)] = (uint16_t)(v[o] >= 1 ? v[o] - 1 : 0);
         }
     }
     const size_t stride = sp.nc2;
@@ -1364,7 +1377,7 @@ __device__ __forceinline__ void contact_create_body(const Space &sp, const Space
                         k = kk + 1;
                     }
                 const int s = k + rem;
-                const double c = r1[k * kTC + t] * ((s == k) ? sq[vb[k * kTC + t]] : r1[s * kTC + t]);
+                const double c = r1[k * kTC + t] * ((s == k) ? sq[vb[vcol(k, t)]] : r1[s * kTC + t]);
                 const uint32_t mm = Xr[k * kTC + t] - Yr[s * kTC + t];
                 cc[j] = c * u(p);
                 ee[j] = c == 0.0 ? make_double2(0.0, 0.0) : __ldg(S + (size_t)(k + s) * stride + mm);
@@ -1410,8 +1423,7 @@ cudaError_t contact_apply_m(const Space &sp, const SpaceTables &tb, const PairOp
     if ((stages & 1) && m1 > m0)
         e = launch_pdl(k_contact_sum<M>, (m1 - m0 + kT2 - 1) / kT2, kT2, tab, st, sp, tb, cv, psi, S, m0, m1);
     if ((stages & 2) && row1 > row0) {
-        const size_t sm = (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + ((M * kTC + 15) & ~15) +
-                          sizeof(double2) * M + tab;
+        const size_t sm = create_smem(M) + tab;
         if (sm > 48 * 1024) {
             if (e == cudaSuccess)
                 e = cudaFuncSetAttribute(k_contact_create<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -1537,8 +1549,8 @@ __global__ void __launch_bounds__(kTC, 3)
     double *r1 = reinterpret_cast<double *>(smem_raw);             // M x kTC
     uint32_t *Xr = reinterpret_cast<uint32_t *>(r1 + M * kTC);     // M x kTC
     uint32_t *Yr = Xr + M * kTC;                                   // M x kTC
-    unsigned char *vb = reinterpret_cast<unsigned char *>(Yr + M * kTC);   // M x kTC
-    double2 *hd = reinterpret_cast<double2 *>(vb + ((M * kTC + 15) & ~15)); // M
+    uint16_t *vb = reinterpret_cast<uint16_t *>(Yr + M * kTC);     // (M + 1) / 2 x 2 kTC (vcol)
+    double2 *hd = reinterpret_cast<double2 *>(vb + (M + 1) / 2 * 2 * kTC); // M
     double *sq = reinterpret_cast<double *>(hd + M);               // wstride
     uint32_t *W = reinterpret_cast<uint32_t *>(sq + sp.wstride);   // (M-1) x wstride
     __shared__ int s_item[2];
@@ -1677,8 +1689,7 @@ cudaError_t fused_apply_m(const Space &sp, const SpaceTables &tb, const PairOp &
                           double2 *E, double2 *out, cudaStream_t st)
 {
     const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
-    const size_t sm = (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + ((M * kTC + 15) & ~15) +
-                      sizeof(double2) * M + tab;
+    const size_t sm = create_smem(M) + tab;
     if (sm > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_hpsi_fused<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
@@ -1694,8 +1705,7 @@ template <int M>
 cudaError_t fused_config_m(const Space &sp, int *grid, size_t *smem)
 {
     const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
-    const size_t sm = (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + ((M * kTC + 15) & ~15) +
-                      sizeof(double2) * M + tab;
+    const size_t sm = create_smem(M) + tab;
     const void *fn = (const void *)k_hpsi_fused<M>;
     cudaError_t e = cudaSuccess;
     if (sm > 48 * 1024 &&
@@ -1986,8 +1996,7 @@ cudaError_t apply_h_m(const Space &sp, const SpaceTables &tb, const PairOp &op, 
         k_pair_annihilate<M><<<g1, kT1, sm1, st>>>(sp, tb, op, psi, E);
     }
     if ((stages & 2) && sp.N >= 2 && op.create_form == 0) {
-        const size_t sm2 = (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + ((M * kTC + 15) & ~15) +
-                           sizeof(double2) * M + tab;
+        const size_t sm2 = create_smem(M) + tab;
         if (sm2 > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(
                 k_pair_create_smem<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm2);
@@ -2183,8 +2192,7 @@ size_t batch_smem(int M, int N, int nh, int stage)
     if (stage == 3)   // the direct form: block values | hd | sqrt products | W | F, G
         return sizeof(double2) * (nh + M) + sizeof(double) * ws * ws + sizeof(uint32_t) * (M - 1) * ws +
                2 * sizeof(uint32_t) * M * kTC;
-    return (sizeof(double) + 2 * sizeof(uint32_t)) * M * kTC + ((M * kTC + 15) & ~15) + sizeof(double2) * M +
-           tab;
+    return create_smem(M) + tab;
 }
 
 int batch_rows_per_block(int stage) { return stage == 1 ? kT2 : kTC; }
