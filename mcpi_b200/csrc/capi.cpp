@@ -41,8 +41,7 @@ int fail(int code, const char *fmt, ...)
     va_start(ap, fmt);
     vsnprintf(buf, sizeof buf, fmt, ap);
     va_end(ap);
-    g_last_error = buf;
-    return code;
+    return mcpi::set_error(code, buf);
 }
 
 #define CK(call)                                                                           \
@@ -552,6 +551,9 @@ static int check_status(mcpi_space_s *sp);
 
 int mcpi::set_error(int code, const char *msg)
 {
+    // a CUDA error that this call reports must not stay pending in the runtime,
+    // where the caller's next launch would find it and fail for it
+    if (code == MCPI_ERR_CUDA || code == MCPI_ERR_NOMEM) (void)cudaGetLastError();
     g_last_error = msg;
     return code;
 }

@@ -880,6 +880,7 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
                                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
                 if (e != cudaSuccess) return e;
                 k_rho1_smem<M, SAME><<<gx, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
+                if (const cudaError_t le = cudaGetLastError(); le != cudaSuccess) return le;
                 return launch_pdl(k_gram_finish<M, 1, SAME ? 3 : 0>, finish, 1024, 0, st, partial, (int)gx, out);
             }
         };
@@ -939,11 +940,10 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
         if (e != cudaSuccess) return e;
         k_gram<M, ORDER, false><<<grid, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
     }
-    if (same)
-        return launch_pdl(k_gram_finish<M, ORDER, 1>, finish, 1024, 0, st, partial, (int)gx, out);
-    else
-        return launch_pdl(k_gram_finish<M, ORDER, 0>, finish, 1024, 0, st, partial, (int)gx, out);
-    return cudaGetLastError();
+    // the finish reports its own launch only: without the partials it must not run
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (same) return launch_pdl(k_gram_finish<M, ORDER, 1>, finish, 1024, 0, st, partial, (int)gx, out);
+    return launch_pdl(k_gram_finish<M, ORDER, 0>, finish, 1024, 0, st, partial, (int)gx, out);
 }
 
 }  // namespace

@@ -1995,6 +1995,8 @@ cudaError_t apply_h_m(const Space &sp, const SpaceTables &tb, const PairOp &op, 
         const unsigned g1 = (sp.nc2 + kT1 - 1) / kT1;
         k_pair_annihilate<M><<<g1, kT1, sm1, st>>>(sp, tb, op, psi, E);
     }
+    // kernel 2 reports its own launch only: without E it must not run
+    if (const cudaError_t e = cudaGetLastError(); e != cudaSuccess) return e;
     if ((stages & 2) && sp.N >= 2 && op.create_form == 0) {
         const size_t sm2 = create_smem(M) + tab;
         if (sm2 > 48 * 1024) {

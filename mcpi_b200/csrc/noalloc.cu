@@ -188,5 +188,7 @@ extern "C" MCPI_API int mcpi_apply_h_static(int N, int M, const double *h_Ho, co
     const mcpi::BlockOp bo{nullptr, 0};
     e = mcpi::launch_apply_h(sp, tb, op, bo, static_cast<const double2 *>(d_C),
                              reinterpret_cast<double2 *>(base + oE), static_cast<double2 *>(d_out), st);
-    return e == cudaSuccess ? MCPI_OK : MCPI_ERR_CUDA;
+    if (e == cudaSuccess) return MCPI_OK;
+    (void)cudaGetLastError();   // reported here: the caller's next launch must not find it
+    return MCPI_ERR_CUDA;
 }

@@ -1,0 +1,86 @@
+"""Host code of the library without a GPU (tests/fake_cuda.py): a launch that
+fails fails the call it belongs to."""
+import pytest
+
+import fake_cuda
+import mcpi_b200 as mc
+from fake_cuda import ERR_CUDA, OK
+
+
+@pytest.fixture(scope="session")
+def fake_so(tmp_path_factory):
+    return fake_cuda.build(tmp_path_factory.mktemp("fake"))
+
+
+@pytest.fixture
+def fake(fake_so):
+    f = fake_cuda.Fake(fake_so)
+    f.reset()
+    yield f
+    f.reset()
+
+
+def every_launch_counts(fake, make, call, most=24):
+    """Fails each launch of a call in turn, on a fresh space (whose first call
+    also builds what the space keeps) and on a used one: the call has to report
+    it, and the next call has to run clean and whole."""
+    s = make()
+    first = fake.kernels(lambda: call(s))
+    warm = fake.kernels(lambda: call(s))
+    assert warm
+    for k in range(min(len(warm), most)):
+        fake.L.fake_fail_launch(k)
+        assert call(s) == ERR_CUDA, k
+        assert fake.kernels(lambda: call(s)) == warm, k
+    s.close()
+    for k in range(min(len(first), most)):
+        s = make()
+        fake.L.fake_fail_launch(k)
+        assert call(s) == ERR_CUDA, k
+        assert set(warm) <= set(fake.kernels(lambda: call(s))) <= set(first) | set(warm), k
+        assert fake.kernels(lambda: call(s)) == warm, k
+        s.close()
+
+
+CALLS = {
+    "apply_h": lambda s: s.apply_h(), "adjoint": lambda s: s.apply_h_adjoint(),
+    "rho1": lambda s: s.density(1), "rho2": lambda s: s.density(2), "t1": lambda s: s.density(1, False),
+    "t2": lambda s: s.density(2, False), "rows": lambda s: s.rows(1, s.nc - 1), "dot": lambda s: s.dot(),
+    "lanczos": lambda s: s.lanczos(9), "ground": lambda s: s.ground(9), "lowmem": lambda s: s.ground(5, True)}
+
+
+# (options, shared memory a block may take): every form of H.psi, and the
+# densities' forms by the orbital count
+@pytest.mark.parametrize("N,M,kind,opts,optin", [
+    (5, 6, "lieb", {}, 0), (5, 6, "lieb", {mc.OPT_DIRECT_HPSI: 0}, 0), (5, 6, "lieb", {mc.OPT_CREATE_FORM: 1}, 0),
+    (5, 6, "lieb", {mc.OPT_DIRECT_HPSI: 0, mc.OPT_FUSED_HPSI: 1}, 0),
+    (5, 6, "lieb", {mc.OPT_NO_MOMENTUM_KERNEL: 1}, 0), (5, 6, "random", {}, 0),
+    (5, 6, "random", {mc.OPT_NO_GEMM_KERNEL: 1}, 0), (4, 10, "random", {}, 120000),
+    (3, 13, "lieb", {}, 0), (3, 16, "random", {}, 0), (70, 2, "lieb", {}, 0)])
+@pytest.mark.parametrize("call", CALLS)
+def test_a_failed_launch_fails_its_call(fake, N, M, kind, opts, optin, call):
+    if optin:
+        fake.L.fake_optin(optin)
+    if call == "rows" and opts.get(mc.OPT_CREATE_FORM):
+        return                                            # row ranges need the default pair-creation form
+    _, Ho, Hint = mc.random_problem(N, M, 3)
+
+    def make():
+        s = fake.space(N, M)
+        for o, v in opts.items():
+            s.option(o, v)
+        assert s.set_integrals(*((Ho, Hint) if kind == "random" else mc.lieb_integrals(M, 1.0))) == OK
+        return s
+
+    every_launch_counts(fake, make, CALLS[call])
+
+
+def test_a_failed_launch_fails_the_batch(fake):
+    b = fake.batch([(4, 7), (5, 7), (3, 10), (4, 10), (3, 12)], 5, mc.lieb_integrals)
+    n = len(fake.kernels(b.run))
+    b.close()
+    for k in range(0, n, 3):
+        b = fake.batch([(4, 7), (5, 7), (3, 10), (4, 10), (3, 12)], 5, mc.lieb_integrals)
+        fake.L.fake_fail_launch(k)
+        assert b.run() == ERR_CUDA, k
+        b.close()
