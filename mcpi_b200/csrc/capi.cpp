@@ -995,8 +995,14 @@ int mcpi_set_integrals(mcpi_space sp, const double *h_Ho, const double *h_Hint, 
             mcpi::Space s2 = sp->sp;
             s2.N = sp->N - 2;
             s2.nc = (uint32_t)sp->nc2;
-            CK(mcpi::launch_pack_occ(sp->sp, t, sp->d_occ, bits, sp->stream));
-            CK(mcpi::launch_pack_occ(s2, t, sp->d_occ2, bits, sp->stream));
+            cudaError_t e = mcpi::launch_pack_occ(sp->sp, t, sp->d_occ, bits, sp->stream);
+            if (e == cudaSuccess) e = mcpi::launch_pack_occ(s2, t, sp->d_occ2, bits, sp->stream);
+            if (e != cudaSuccess) {   // no table is left that was not written
+                cudaFree(sp->d_occ);
+                cudaFree(sp->d_occ2);
+                sp->d_occ = sp->d_occ2 = nullptr;
+                CK(e);
+            }
             sp->occ_bits = bits;
         } else {
             (void)cudaGetLastError();
@@ -1179,8 +1185,13 @@ static int density(mcpi_space sp, int order, const void *phi, const void *psi, v
             mcpi::Space s1 = sp->sp;
             s1.N = sp->N - 1;
             s1.nc = (uint32_t)sp->nc1;
-            CK(mcpi::launch_pack_occ(s1, mcpi::SpaceTables{sp->d_W, sp->d_sq}, sp->d_occ1, sp->occ_bits,
-                                     sp->stream));
+            const cudaError_t e = mcpi::launch_pack_occ(s1, mcpi::SpaceTables{sp->d_W, sp->d_sq}, sp->d_occ1,
+                                                        sp->occ_bits, sp->stream);
+            if (e != cudaSuccess) {
+                cudaFree(sp->d_occ1);
+                sp->d_occ1 = nullptr;
+                CK(e);
+            }
         } else {
             (void)cudaGetLastError();
             sp->d_occ1 = nullptr;

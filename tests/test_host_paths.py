@@ -84,3 +84,17 @@ def test_a_failed_launch_fails_the_batch(fake):
         fake.L.fake_fail_launch(k)
         assert b.run() == ERR_CUDA, k
         b.close()
+
+
+def test_a_failed_table_launch_leaves_no_table(fake):
+    # mcpi_set_integrals packs the occupations of two spaces, the first rho1 of a third
+    for k in range(2):
+        s = fake.space(5, 6)
+        fake.L.fake_fail_launch(k)
+        assert s.set_integrals(*mc.lieb_integrals(6, 1.0)) == ERR_CUDA
+        again = fake.kernels(lambda: s.set_integrals(*mc.lieb_integrals(6, 1.0)))
+        assert len([n for n in again if "k_pack_occ" in n]) == 2
+        fake.L.fake_fail_launch(0)
+        assert s.density(1) == ERR_CUDA
+        assert len([n for n in fake.kernels(lambda: s.density(1)) if "k_pack_occ" in n]) == 1
+        s.close()
