@@ -385,32 +385,43 @@ int ensure_E(mcpi_space_s *sp, const PairOp &v)
     return ensure_fused(sp);
 }
 
-// One H.psi on the space's stream.
-cudaError_t run_hpsi(mcpi_space_s *sp, const DevPairOp &op, PairOp &v, const double2 *psi, double2 *out,
-                     int stages = 3, uint32_t row0 = 0, uint32_t row1 = 0xffffffffu, uint32_t m0 = 0,
-                     uint32_t m1 = 0xffffffffu)
-{
-    const cudaStream_t st = sp->stream;
-    double2 *scratch = sp->d_E;
-    void *S = nullptr;
-    if (mcpi::hpsi_form(sp->sp, v) == mcpi::kFormContact) {
-        scratch = sp->d_S;
-        if (mcpi::direct_covers(sp->sp)) {
-            if (contact_bytes(sp) > mcpi::kContactMaxBytes ||
-                pool_alloc(sp->device, &S, contact_bytes(sp), st) != cudaSuccess) {
-                (void)cudaGetLastError();
-                v.contact = nullptr;   // the direct form
-            }
-            scratch = (double2 *)S;
+// What H.psi in the form of v passes between its halves, held as long as this
+// object lives: the space's E or S, or an S from the pool. Where the pool has
+// none, v becomes the direct form. A solve holds one, so that all its H.psi take
+// one form (two forms round differently, and the second pass of
+// mcpi_ground_lowmem has to meet the first one's vectors bit for bit).
+struct HpsiScratch {
+    double2 *ptr;
+    void *pool = nullptr;
+    cudaStream_t st;
+    HpsiScratch(mcpi_space_s *sp, PairOp &v) : ptr(sp->d_E), st(sp->stream)
+    {
+        if (mcpi::hpsi_form(sp->sp, v) != mcpi::kFormContact) return;
+        ptr = sp->d_S;
+        if (!mcpi::direct_covers(sp->sp)) return;
+        if (contact_bytes(sp) > mcpi::kContactMaxBytes ||
+            pool_alloc(sp->device, &pool, contact_bytes(sp), st) != cudaSuccess) {
+            (void)cudaGetLastError();
+            pool = nullptr;
+            v.contact = nullptr;   // the direct form
         }
+        ptr = (double2 *)pool;
     }
-    cudaError_t e = mcpi::launch_apply_h(sp->sp, sp->tables(), v, op.blocks(), psi, scratch, out, st, stages, row0,
-                                         row1, m0, m1);
-    if (S) {
-        const cudaError_t f = cudaFreeAsync(S, st);
-        if (e == cudaSuccess) e = f;
+    ~HpsiScratch()
+    {
+        if (pool && cudaFreeAsync(pool, st) != cudaSuccess) (void)cudaGetLastError();
     }
-    return e;
+    HpsiScratch(const HpsiScratch &) = delete;
+    HpsiScratch &operator=(const HpsiScratch &) = delete;
+};
+
+// One H.psi on the space's stream, in the form that v has once its scratch is taken.
+cudaError_t run_hpsi(mcpi_space_s *sp, const DevPairOp &op, const PairOp &v, const HpsiScratch &scratch,
+                     const double2 *psi, double2 *out, int stages = 3, uint32_t row0 = 0,
+                     uint32_t row1 = 0xffffffffu, uint32_t m0 = 0, uint32_t m1 = 0xffffffffu)
+{
+    return mcpi::launch_apply_h(sp->sp, sp->tables(), v, op.blocks(), psi, scratch.ptr, out, sp->stream, stages, row0,
+                                row1, m0, m1);
 }
 
 int reserve(mcpi_space_s *sp, void *&ptr, size_t &cap, size_t bytes)
@@ -537,7 +548,8 @@ int apply_op(mcpi_space_s *sp, const DevPairOp &op, const void *d_C, void *d_out
     int rc = ensure_E(sp, v);
     if (rc) return rc;
     if (sp->fz_ready) v = op_view(sp, op);   // the schedule that ensure_E may have built
-    CK(run_hpsi(sp, op, v, (const double2 *)d_C, (double2 *)d_out));
+    const HpsiScratch scratch(sp, v);
+    CK(run_hpsi(sp, op, v, scratch, (const double2 *)d_C, (double2 *)d_out));
     return MCPI_OK;
 }
 
@@ -1037,6 +1049,7 @@ int mcpi_apply_h_host(mcpi_space sp, int count, const void *const *h_C, void *co
         CK(e);
     }
     fop = op_view(sp, sp->fwd);
+    const HpsiScratch scratch(sp, fop);
     // buffer pair b = k & 1: its input is free once H.psi of state k-2 has run,
     // its output once the copy out of state k-2 has finished
     for (int k = 0; k < count; ++k) {
@@ -1046,7 +1059,7 @@ int mcpi_apply_h_host(mcpi_space sp, int count, const void *const *h_C, void *co
         CK(cudaEventRecord(sp->ev_in[b], sp->s_h2d));
         CK(cudaStreamWaitEvent(sp->stream, sp->ev_in[b], 0));
         if (k >= 2) CK(cudaStreamWaitEvent(sp->stream, sp->ev_out[b], 0));
-        CK(run_hpsi(sp, sp->fwd, fop, sp->d_hin[b], sp->d_hout[b]));
+        CK(run_hpsi(sp, sp->fwd, fop, scratch, sp->d_hin[b], sp->d_hout[b]));
         CK(cudaEventRecord(sp->ev_comp[b], sp->stream));
         CK(cudaStreamWaitEvent(sp->s_d2h, sp->ev_comp[b], 0));
         CK(cudaMemcpyAsync(h_out[k], sp->d_hout[b], bytes, cudaMemcpyDeviceToHost, sp->s_d2h));
@@ -1070,20 +1083,7 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
     for (auto &e : ev) CK(cudaEventCreate(&e));
     float tot[2] = {0.f, 0.f};
     cudaError_t e = cudaSuccess;
-    // the contact form's two halves run apart here, on one S
-    double2 *scratch = sp->d_E;
-    void *S = nullptr;
-    if (mcpi::hpsi_form(sp->sp, fop) == mcpi::kFormContact) {
-        scratch = sp->d_S;
-        if (mcpi::direct_covers(sp->sp)) {
-            if (contact_bytes(sp) > mcpi::kContactMaxBytes ||
-                pool_alloc(sp->device, &S, contact_bytes(sp), sp->stream) != cudaSuccess) {
-                (void)cudaGetLastError();
-                fop.contact = nullptr;
-            }
-            scratch = (double2 *)S;
-        }
-    }
+    const HpsiScratch scratch(sp, fop);   // the two halves run apart here, on one scratch
     const int form = mcpi::hpsi_form(sp->sp, fop);
     const bool one = form == mcpi::kFormDirect || form == mcpi::kFormFused;
     if (one) {
@@ -1091,7 +1091,7 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
         for (int r = 0; r < reps && e == cudaSuccess; ++r) {
             e = cudaEventRecord(ev[0], sp->stream);
             if (e == cudaSuccess)
-                e = run_hpsi(sp, sp->fwd, fop, (const double2 *)d_C, (double2 *)d_out);
+                e = run_hpsi(sp, sp->fwd, fop, scratch, (const double2 *)d_C, (double2 *)d_out);
             if (e == cudaSuccess) e = cudaEventRecord(ev[1], sp->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(ev[1]);
             float a = 0.f;
@@ -1102,12 +1102,10 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
     for (int r = 0; r < reps && e == cudaSuccess && !one; ++r) {
         e = cudaEventRecord(ev[0], sp->stream);
         if (e == cudaSuccess)
-            e = mcpi::launch_apply_h(sp->sp, sp->tables(), fop, sp->fwd.blocks(), (const double2 *)d_C, scratch,
-                                     (double2 *)d_out, sp->stream, 1);
+            e = run_hpsi(sp, sp->fwd, fop, scratch, (const double2 *)d_C, (double2 *)d_out, 1);
         if (e == cudaSuccess) e = cudaEventRecord(ev[1], sp->stream);
         if (e == cudaSuccess)
-            e = mcpi::launch_apply_h(sp->sp, sp->tables(), fop, sp->fwd.blocks(), (const double2 *)d_C, scratch,
-                                     (double2 *)d_out, sp->stream, 2);
+            e = run_hpsi(sp, sp->fwd, fop, scratch, (const double2 *)d_C, (double2 *)d_out, 2);
         if (e == cudaSuccess) e = cudaEventRecord(ev[2], sp->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(ev[2]);
         float a = 0.f, b = 0.f;
@@ -1117,7 +1115,6 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
         tot[1] += b;
     }
     for (auto &x : ev) cudaEventDestroy(x);
-    if (S) cudaFreeAsync(S, sp->stream);
     if (e != cudaSuccess) return fail(MCPI_ERR_CUDA, "mcpi_apply_h_profile: %s", cudaGetErrorString(e));
     h_ms[0] = tot[0] / reps;
     h_ms[1] = tot[1] / reps;
@@ -1163,7 +1160,9 @@ int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1
         m0 = sp->mr_lo;
         m1 = sp->mr_hi + 1;
     }
-    CK(run_hpsi(sp, sp->fwd, fop, (const double2 *)d_C, (double2 *)d_out, 3, (uint32_t)row0, (uint32_t)row1, m0, m1));
+    const HpsiScratch scratch(sp, fop);
+    CK(run_hpsi(sp, sp->fwd, fop, scratch, (const double2 *)d_C, (double2 *)d_out, 3, (uint32_t)row0, (uint32_t)row1,
+                m0, m1));
     return MCPI_OK;
 }
 
@@ -1348,17 +1347,18 @@ int mcpi_lanczos(mcpi_space sp, void *d_lvec, int lm, double *h_diag, double *h_
             one_launch = false;
         }
     }
-    if (!one_launch) {
-        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, V, r);
+    if (!one_launch && e == cudaSuccess) {
+        const HpsiScratch scratch(sp, op);
+        e = run_hpsi(sp, sp->fwd, op, scratch, V, r);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_start(V, r, r, nc, s, sp->stream);
-    }
-    for (int i = 0; i < lm - 1 && e == cudaSuccess && !one_launch; ++i) {
-        double2 *vi = V + (size_t)i * nc, *vn = V + (size_t)(i + 1) * nc;
-        e = mcpi::launch_lanczos_beta(i, lm, 1e-15, s, sp->stream);
-        if (e == cudaSuccess) e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, sp->stream);
-        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, vn, r);
-        if (e == cudaSuccess) e = mcpi::launch_lanczos_alpha(vi, vn, r, nc, i, s, sp->stream);
-        if (e == cudaSuccess) e = mcpi::launch_lanczos_reorth(V, i + 2, r, nc, i, s, sp->stream);
+        for (int i = 0; i < lm - 1 && e == cudaSuccess; ++i) {
+            double2 *vi = V + (size_t)i * nc, *vn = V + (size_t)(i + 1) * nc;
+            e = mcpi::launch_lanczos_beta(i, lm, 1e-15, s, sp->stream);
+            if (e == cudaSuccess) e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, sp->stream);
+            if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, scratch, vn, r);
+            if (e == cudaSuccess) e = mcpi::launch_lanczos_alpha(vi, vn, r, nc, i, s, sp->stream);
+            if (e == cudaSuccess) e = mcpi::launch_lanczos_reorth(V, i + 2, r, nc, i, s, sp->stream);
+        }
     }
     std::vector<double2> alpha(lm);
     std::vector<double> beta(lm);
@@ -1460,17 +1460,18 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     op = lanczos_view(sp);
     const int init[2] = {0, lm};
     cudaStream_t st = sp->stream;
+    const HpsiScratch scratch(sp, op);   // of both passes
     // pass 1: tridiagonal only
     e = cudaMemsetAsync(blk, 0, sbytes, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s.done, init, sizeof init, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(v[0], d_C, sizeof(double2) * nc, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, v[0], r);
+    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, scratch, v[0], r);
     if (e == cudaSuccess) e = mcpi::launch_lanczos_start(v[0], r, r, nc, s, st);
     for (int i = 0; i < lm - 1 && e == cudaSuccess; ++i) {
         double2 *vi = v[i & 1], *vn = v[(i + 1) & 1];
         e = mcpi::launch_lanczos_beta(i, lm, 1e-15, s, st);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, st);
-        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, vn, r);
+        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, scratch, vn, r);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_alpha(vi, vn, r, nc, i, s, st);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_no_reorth(vn, r, nc, i, s, st);
     }
@@ -1497,13 +1498,13 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     if (e == cudaSuccess) e = cudaMemcpyAsync(dz, zc.data(), sizeof(double) * lm, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(s.done, init, sizeof init, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(v[0], d_C, sizeof(double2) * nc, cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, v[0], r);
+    if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, scratch, v[0], r);
     if (e == cudaSuccess) e = mcpi::launch_lanczos_no_reorth(v[0], r, nc, -1, s, st);
     if (e == cudaSuccess) e = mcpi::launch_axpy_real(acc, v[0], nc, dz, 1, st);
     for (int i = 0; i < n - 1 && e == cudaSuccess; ++i) {
         double2 *vi = v[i & 1], *vn = v[(i + 1) & 1];
         e = mcpi::launch_lanczos_scale(r, vn, nc, i, s, st);
-        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, vn, r);
+        if (e == cudaSuccess) e = run_hpsi(sp, sp->fwd, op, scratch, vn, r);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_axpy(vi, r, nc, i, s, st);
         if (e == cudaSuccess) e = mcpi::launch_lanczos_no_reorth(vn, r, nc, i, s, st);
         if (e == cudaSuccess) e = mcpi::launch_axpy_real(acc, vn, nc, dz + i + 1, 0, st);

@@ -98,3 +98,26 @@ def test_a_failed_table_launch_leaves_no_table(fake):
         assert s.density(1) == ERR_CUDA
         assert len([n for n in fake.kernels(lambda: s.density(1)) if "k_pack_occ" in n]) == 1
         s.close()
+
+
+def forms(kernels):
+    """The forms of H.psi among the launched kernels."""
+    known = {"k_contact_sum": "contact", "k_hpsi_direct": "direct", "k_pair_create": "pairs", "k_hpsi_fused": "fused"}
+    return {f for k, f in known.items() for n in kernels if k in n}
+
+
+@pytest.mark.parametrize("lowmem", [False, True])
+def test_a_solve_keeps_one_form_when_memory_runs_out(fake, lowmem):
+    # N=12, M=10: contact form with an S from the pool. Whichever of its requests
+    # the pool turns down, once or for good, all H.psi of a solve take one form.
+    s = fake.space(12, 10)
+    assert s.set_integrals(*mc.lieb_integrals(10, 1.0)) == OK
+    solve = (lambda: s.ground(6, True)) if lowmem else (lambda: s.lanczos(6))
+    assert forms(fake.kernels(solve)) == {"contact"}
+    for for_good in (0, 1):
+        for k in range(12):
+            fake.L.fake_fail_pool(k, for_good)
+            got = forms(fake.kernels(solve))
+            assert got == {"direct" if k == 0 else "contact"}, (for_good, k)
+            fake.L.fake_fail_pool(-1, 0)
+    s.close()
