@@ -207,13 +207,18 @@ MCPI_API int mcpi_dot(mcpi_space sp, const void *d_a, const void *d_b, double *h
  * shard) and runs the reference's recurrence with these calls, summing each
  * per-rank result (dot, coefficients, norm^2) over the ranks with an
  * all-reduce between the calls (mcpi_b200/distributed.py is the driver; the
- * H.psi of a shard is mcpi_apply_h_rows on the all-gathered vector). All
+ * H.psi of a shard is mcpi_shard_apply_h on the all-gathered vector). All
  * scalars stay in device memory, so a solve needs no host round trip; every
  * kernel returns at entry once *d_done != 0, so all ranks keep issuing the
  * same collectives after a breakdown. Sums inside a rank run in a fixed
  * order. Device pointers (complex = 2 doubles), work on `stream`.
  *   scratch: mcpi_shard_scratch_elems(n, lm) complex entries. */
 MCPI_API size_t mcpi_shard_scratch_elems(int64_t n, int lm);
+/* mcpi_apply_h_rows in the form that mcpi_lanczos takes, on the space's stream: the
+ * two differ for contact interactions of an odd number of plane waves, where the
+ * recurrence amplifies rounding to order one. On one rank (the whole range) the
+ * solve is then mcpi_lanczos bit for bit. */
+MCPI_API int mcpi_shard_apply_h(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1, void *d_out);
 /* vnext = r / *beta_i */
 MCPI_API int mcpi_shard_scale(int64_t n, const void *d_r, void *d_vnext, const double *d_beta_i,
                               const int *d_done, void *stream);

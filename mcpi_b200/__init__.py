@@ -22,6 +22,7 @@ from __future__ import annotations
 
 import ctypes as ct
 import os
+import threading
 
 import numpy as np
 
@@ -88,6 +89,7 @@ def lib():
         "mcpi_apply_h": (i, [_vp, _vp, _vp]),
         "mcpi_apply_h_adjoint": (i, [_vp, _vp, _vp]),
         "mcpi_apply_h_rows": (i, [_vp, _vp, i64, i64, _vp]),
+        "mcpi_shard_apply_h": (i, [_vp, _vp, i64, i64, _vp]),
         "mcpi_apply_h_host": (i, [_vp, i, _vp, _vp]),
         "mcpi_apply_h_profile": (i, [_vp, _vp, _vp, i, _vp]),
         "mcpi_rho1": (i, [_vp, _vp, _vp]),
@@ -193,6 +195,10 @@ def tridiag_eig(d, e, vectors: bool = True):
 def _torch():
     import torch
     return torch
+
+
+# per thread: whether row ranges belong to a sharded solve (distributed.solve_rows)
+_rows = threading.local()
 
 
 class FockSpace:
@@ -329,12 +335,13 @@ class FockSpace:
         return outs
 
     def apply_h_rows(self, C, row0: int, row1: int, out=None):
-        """Rows [row0, row1) of H C (C the whole vector)."""
+        """Rows [row0, row1) of H C (C the whole vector). Inside solve_rows() in the
+        form that `lanczos` takes (mcpi_shard_apply_h)."""
         C = self._vec(C)
         out = self.empty(row1 - row0) if out is None else out
         self._stream()
-        _check(lib().mcpi_apply_h_rows(self._h, _vp(C.data_ptr()), row0, row1,
-                                       _vp(out.data_ptr()) if row1 > row0 else None))
+        f = lib().mcpi_shard_apply_h if getattr(_rows, "solve", False) else lib().mcpi_apply_h_rows
+        _check(f(self._h, _vp(C.data_ptr()), row0, row1, _vp(out.data_ptr()) if row1 > row0 else None))
         return out
 
     def apply_h_profile(self, C, out=None, reps: int = 10):

@@ -1121,12 +1121,13 @@ int mcpi_apply_h_profile(mcpi_space sp, const void *d_C, void *d_out, int reps, 
     return MCPI_OK;
 }
 
-int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1, void *d_out)
+// Rows [row0, row1) of H C: in the form of a single H.psi, or of a solve's.
+static int apply_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1, void *d_out, bool solve)
 {
-    CHECK_ARG(sp && d_C && d_C != d_out, "mcpi_apply_h_rows: bad arguments");
-    CHECK_ARG(row0 >= 0 && row0 <= row1 && row1 <= sp->nc, "mcpi_apply_h_rows: bad row range");
+    CHECK_ARG(sp && d_C && d_C != d_out, "row range of H.psi: bad arguments");
+    CHECK_ARG(row0 >= 0 && row0 <= row1 && row1 <= sp->nc, "row range of H.psi: bad row range");
     if (row0 == row1) return MCPI_OK;
-    CHECK_ARG(d_out, "mcpi_apply_h_rows: null output");
+    CHECK_ARG(d_out, "row range of H.psi: null output");
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     if (sp->N < 2 || sp->create_form != 0)
         return fail(MCPI_ERR_ARG, "row ranges need N >= 2 and the default pair-creation form");
@@ -1135,11 +1136,12 @@ int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1
     // exactly the rows', while the contact form's first half covers every
     // configuration that they read
     const bool part = row0 != 0 || row1 != sp->nc;
-    PairOp fop = op_view(sp, sp->fwd);
+    auto view = [&] { return solve ? lanczos_view(sp) : op_view(sp, sp->fwd); };
+    PairOp fop = view();
     if (part && mcpi::direct_covers(sp->sp)) fop.contact = nullptr;
     int rc = ensure_E(sp, fop);
     if (rc) return rc;
-    if (sp->fz_ready) fop = op_view(sp, sp->fwd);
+    if (sp->fz_ready) fop = view();
     // kernel 1 only over the E columns these rows read (momentum-block form):
     // a rank of a sharded solve does not recompute the whole intermediate.
     // The range is found once per row block (one pass over its rows).
@@ -1164,6 +1166,16 @@ int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1
     CK(run_hpsi(sp, sp->fwd, fop, scratch, (const double2 *)d_C, (double2 *)d_out, 3, (uint32_t)row0, (uint32_t)row1,
                 m0, m1));
     return MCPI_OK;
+}
+
+int mcpi_apply_h_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1, void *d_out)
+{
+    return apply_rows(sp, d_C, row0, row1, d_out, false);
+}
+
+int mcpi_shard_apply_h(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1, void *d_out)
+{
+    return apply_rows(sp, d_C, row0, row1, d_out, true);
 }
 
 int mcpi_apply_h_adjoint(mcpi_space sp, const void *d_C, void *d_out)

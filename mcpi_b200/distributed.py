@@ -5,7 +5,8 @@ rank stores only its rows of every Krylov vector. Per Lanczos step:
 
 * all-gather of the new Krylov vector (every rank needs the whole vector: an
   H.psi row gathers from anywhere in the space);
-* local H.psi of the owned rows (`mcpi_apply_h_rows` on the GPU);
+* local H.psi of the owned rows (`mcpi_shard_apply_h` on the GPU: in the form that
+  `mcpi_lanczos` takes, see `solve_rows`);
 * all-reduce of this rank's alpha dot, of its reorthogonalisation
   coefficients V^H r and of its residual norm^2.
 
@@ -23,13 +24,14 @@ the kernels and an injected local operator.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as ct
 
 import numpy as np
 import torch
 import torch.distributed as dist
 
-from . import MCPIError, lib, tridiag_eig
+from . import MCPIError, _rows, lib, tridiag_eig
 
 _vp = ct.c_void_p
 
@@ -39,6 +41,21 @@ def row_block(nc: int, world: int, rank: int):
     base, extra = divmod(nc, world)
     r0 = rank * base + min(rank, extra)
     return r0, r0 + base + (1 if rank < extra else 0)
+
+
+@contextlib.contextmanager
+def solve_rows():
+    """Inside, `FockSpace.apply_h_rows` on this thread is `mcpi_shard_apply_h`: the
+    rows in the form that `mcpi_lanczos` takes. A single H.psi may take another
+    one (contact interactions of an odd number of plane waves), and there the
+    recurrence amplifies rounding to order one. ShardedLanczos applies its local
+    operator inside."""
+    before = getattr(_rows, "solve", False)
+    _rows.solve = True
+    try:
+        yield
+    finally:
+        _rows.solve = before
 
 
 def _p(t):
@@ -181,6 +198,10 @@ class ShardedLanczos:
         """In-place all-reduce of a device scalar or vector (complex as pairs)."""
         dist.all_reduce(torch.view_as_real(t) if t.is_complex() else t, group=self.group)
 
+    def _apply(self, v):
+        with solve_rows():
+            return self.local_apply(v)
+
     # Lanczos ----------------------------------------------------------------
     def lanczos(self, v0_shard, lm: int, tol: float = 1e-15):
         """Returns (iterations, alpha[lm] complex, beta[lm], Krylov shards [lm, r1-r0])."""
@@ -198,7 +219,7 @@ class ShardedLanczos:
         send = torch.zeros(self.maxb, dtype=torch.complex128, device=dev)
         gbuf = torch.empty(self.world * self.maxb, dtype=torch.complex128, device=dev)
 
-        r = self.local_apply(self._gather(V[0], send, gbuf))
+        r = self._apply(self._gather(V[0], send, gbuf))
         ops.axpy_dot(None, V[0], r, None, alpha[0:1], done)          # alpha_0 = <v0, H v0>
         self._sum(alpha[0:1])
         ops.update(None, 0, r, V[0], alpha[0:1], None, norm2, done)  # r -= alpha_0 v0
@@ -206,7 +227,7 @@ class ShardedLanczos:
         for i in range(lm - 1):
             ops.beta(i, tol, norm2, beta, maxb, done, iters)
             ops.scale(r, V[i + 1], beta[i:i + 1], done)
-            r = self.local_apply(self._gather(V[i + 1], send, gbuf))
+            r = self._apply(self._gather(V[i + 1], send, gbuf))
             ops.axpy_dot(V[i], V[i + 1], r, beta[i:i + 1], alpha[i + 1:i + 2], done)
             self._sum(alpha[i + 1:i + 2])
             ops.multidot(V, i + 2, r, V[i + 1], alpha[i + 1:i + 2], coef, done)

@@ -121,3 +121,42 @@ def test_a_solve_keeps_one_form_when_memory_runs_out(fake, lowmem):
             assert got == {"direct" if k == 0 else "contact"}, (for_good, k)
             fake.L.fake_fail_pool(-1, 0)
     s.close()
+
+
+# (N, M, form of a single H.psi, form of a solve, form of a part of a solve's rows)
+@pytest.mark.parametrize("N,M,single,solve,part", [
+    (10, 11, "contact", "direct", "direct"), (5, 13, "contact", "pairs", "pairs"), (4, 15, "contact", "pairs", "pairs"),
+    (5, 12, "contact", "contact", "contact"), (12, 10, "contact", "contact", "direct"), (6, 9, "direct", "direct", "direct")])
+def test_rows_of_a_solve_take_its_form(fake, N, M, single, solve, part):
+    s = fake.space(N, M)
+    assert s.set_integrals(*mc.lieb_integrals(M, 1.0)) == OK
+    s.option(mc.OPT_FUSED_HPSI, 0)
+    rows = lambda e, r0, r1: forms(fake.kernels(lambda: s.rows(r0, r1, e)))
+    assert forms(fake.kernels(s.apply_h)) == {single} == rows("mcpi_apply_h_rows", 0, s.nc)
+    if s.nc > 13000:                       # smaller ones may take the one-launch Lanczos
+        assert forms(fake.kernels(lambda: s.lanczos(3))) == {solve}
+    assert forms(fake.kernels(lambda: s.ground(3, True))) == {solve}
+    assert rows("mcpi_shard_apply_h", 0, s.nc) == {solve}
+    assert rows("mcpi_shard_apply_h", 5, s.nc // 2) == {part}
+    s.close()
+
+
+def test_solve_rows_is_per_thread_and_nests():
+    import threading
+    from mcpi_b200 import _rows
+    from mcpi_b200.distributed import solve_rows
+    seen = []
+    with solve_rows():
+        with solve_rows():
+            pass
+        seen.append(_rows.solve)
+        t = threading.Thread(target=lambda: seen.append(getattr(_rows, "solve", False)))
+        t.start()
+        t.join()
+        try:
+            with solve_rows():
+                raise KeyError
+        except KeyError:
+            pass
+        seen.append(_rows.solve)
+    assert seen == [True, False, True] and not _rows.solve
