@@ -443,8 +443,14 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
             tot += mcpi::up256(sizeof(double2) * (2 * (size_t)lm + (size_t)(lm + 1) * b->lz[m].ntiles) +
                                sizeof(double) * (lm + 1) + 2 * sizeof(int));
         }
-        if (cudaMalloc(&b->arena, tot) != cudaSuccess) {
+        size_t later = 0, left = 0, all = 0;   // tables, operators and metadata still to come
+        for (const mcpi_space_s *s : b->spaces)
+            later += sizeof(uint64_t) * (size_t)(s->nc + s->nc2) + ((size_t)1 << 20);
+        if (mcpi::device_malloc(device, reinterpret_cast<void **>(&b->arena), tot) != cudaSuccess) {
             (void)cudaGetLastError();
+            b->arena = nullptr;
+        } else if (with_S && (cudaMemGetInfo(&left, &all) != cudaSuccess || left < later)) {
+            cudaFree(b->arena);
             b->arena = nullptr;
         }
         b->has_S = with_S != 0;
@@ -569,7 +575,8 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
         for (size_t c = 0; c < pw1[g].size(); ++c)
             mbytes += mcpi::up256(sizeof(int2) * pw1[g][c].size()) + mcpi::up256(sizeof(int2) * pw2[g][c].size());
     }
-    if (cudaMalloc(&b->meta, mbytes) != cudaSuccess) return cleanup(MCPI_ERR_NOMEM, "metadata allocation failed");
+    if (mcpi::device_malloc(device, reinterpret_cast<void **>(&b->meta), mbytes) != cudaSuccess)
+        return cleanup(MCPI_ERR_NOMEM, "metadata allocation failed");
     char *p = b->meta;
     auto take = [&](size_t bytes) {
         char *q = p;

@@ -94,6 +94,12 @@ struct DeviceGuard {
 
 namespace {
 
+template <class T>
+cudaError_t dev_malloc(const mcpi_space_s *sp, T **ptr, size_t bytes)
+{
+    return mcpi::device_malloc(sp->device, reinterpret_cast<void **>(ptr), bytes);
+}
+
 void free_op(DevPairOp &o)
 {
     cudaFree(o.hblk);
@@ -246,11 +252,11 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
     }
     free_op(op);
     const size_t nnz = col.size() ? col.size() : 1;
-    CK(cudaMalloc(&op.rowptr, sizeof(int) * (P + 1)));
-    CK(cudaMalloc(&op.col, sizeof(uint16_t) * nnz));
-    CK(cudaMalloc(&op.val, sizeof(double2) * nnz));
-    CK(cudaMalloc(&op.hdiag, sizeof(double2) * M));
-    CK(cudaMalloc(&op.hfull, sizeof(double2) * M * M));
+    CK(dev_malloc(sp, &op.rowptr, sizeof(int) * (P + 1)));
+    CK(dev_malloc(sp, &op.col, sizeof(uint16_t) * nnz));
+    CK(dev_malloc(sp, &op.val, sizeof(double2) * nnz));
+    CK(dev_malloc(sp, &op.hdiag, sizeof(double2) * M));
+    CK(dev_malloc(sp, &op.hfull, sizeof(double2) * M * M));
     CK(cudaMemcpyAsync(op.rowptr, rowptr.data(), sizeof(int) * (P + 1), cudaMemcpyHostToDevice, sp->stream));
     if (!col.empty()) {
         CK(cudaMemcpyAsync(op.col, col.data(), sizeof(uint16_t) * col.size(), cudaMemcpyHostToDevice, sp->stream));
@@ -260,7 +266,7 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
     CK(cudaMemcpyAsync(op.hfull, hfull, sizeof(double2) * M * M, cudaMemcpyHostToDevice, sp->stream));
     const std::vector<cplx> mom = pack_momentum(Ht, P, M);
     if (!mom.empty() && !sp->dense_only && sp->kernel_choice != 2) {
-        CK(cudaMalloc(&op.hblk, sizeof(double2) * mom.size()));
+        CK(dev_malloc(sp, &op.hblk, sizeof(double2) * mom.size()));
         CK(cudaMemcpyAsync(op.hblk, mom.data(), sizeof(double2) * mom.size(), cudaMemcpyHostToDevice, sp->stream));
         op.nhblk = (int)mom.size();
         op.hblk_h.resize(mom.size());
@@ -272,7 +278,7 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
     }
     const std::vector<int> prog = pack_blocks(Ht, P, M);
     if (!prog.empty() && !sp->dense_only) {
-        CK(cudaMalloc(&op.prog, sizeof(int) * prog.size()));
+        CK(dev_malloc(sp, &op.prog, sizeof(int) * prog.size()));
         CK(cudaMemcpyAsync(op.prog, prog.data(), sizeof(int) * prog.size(), cudaMemcpyHostToDevice, sp->stream));
         op.prog_bytes = (int)(sizeof(int) * prog.size());
     }
@@ -281,7 +287,7 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
     // nnz at a fraction of it, so the dense form pays once a quarter is filled.
     const bool general = (mom.empty() || sp->kernel_choice == 2) && prog.empty() && 4 * col.size() >= (size_t)P * P;
     if (P <= mcpi::kGemmMaxP && !sp->no_gemm && (sp->dense_only || general)) {
-        CK(cudaMalloc(&op.hdense, sizeof(double2) * P * P));
+        CK(dev_malloc(sp, &op.hdense, sizeof(double2) * P * P));
         CK(cudaMemcpyAsync(op.hdense, Ht.data(), sizeof(double2) * P * P, cudaMemcpyHostToDevice, sp->stream));
     }
     CK(cudaStreamSynchronize(sp->stream));  // host vectors go out of scope
@@ -302,17 +308,19 @@ size_t contact_bytes(const mcpi_space_s *sp)
 }
 
 // Stream-ordered scratch of the contact form on spaces whose calls the direct
-// form, which has no scratch, can take: each call allocates its S and gives it
-// back on its own stream, so calls on several streams or threads stay
-// independent, and a call that finds no memory runs the direct form. One pool
+// form, which has no scratch, can take: each call or solve allocates its S and
+// gives it back on its own stream, so calls on several streams or threads stay
+// independent, and one that finds no memory runs the direct form. One pool
 // per device for all spaces. It keeps at most kContactMaxBytes that no call uses
-// (mapping fresh memory costs milliseconds per GB) and returns those to the
-// device when the last space on the device goes, or when an allocation of
-// the library fails.
+// (mapping fresh memory costs milliseconds per GB). Other allocations get those
+// back: any cudaMalloc of the process does from the driver once the host has seen
+// the calls end (measured; it is the host program's own allocator's way too), the
+// library's after waiting for them (device_malloc), and all of it when the last
+// space on the device goes.
 struct ScratchPool {
-    std::mutex mutex;
+    std::mutex mutex;   // also guards the streams of the listed spaces
     cudaMemPool_t pool[64] = {};
-    int spaces[64] = {};
+    std::vector<const mcpi_space_s *> spaces[64];
 };
 ScratchPool &scratch()
 {
@@ -341,31 +349,42 @@ cudaError_t pool_alloc(int device, void **ptr, size_t bytes, cudaStream_t st)
     return cudaMallocFromPoolAsync(ptr, bytes, pool, st);
 }
 
+// Returns the pool's unused memory to the device, once the calls queued on the
+// spaces' streams have ended: memory freed on a stream counts as used until the
+// host has synchronised with it. (A captured stream is left alone. cudaFree's
+// implicit wait does not count as one, measured.)
 void pool_trim(int device)
 {
     ScratchPool &p = scratch();
     std::lock_guard<std::mutex> lock(p.mutex);
-    if (p.pool[device]) cudaMemPoolTrimTo(p.pool[device], 0);
+    uint64_t held = 0;
+    if (!p.pool[device] ||
+        (cudaMemPoolGetAttribute(p.pool[device], cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess && !held))
+        return;
+    for (const mcpi_space_s *sp : p.spaces[device]) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(sp->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+            cudaStreamSynchronize(sp->stream);
+    }
+    cudaMemPoolTrimTo(p.pool[device], 0);
+    (void)cudaGetLastError();
 }
 
-// Counts the spaces of a device; the pool empties with the last one.
-void pool_space(int device, int step)
+// Lists the spaces of a device; the pool empties with the last one.
+void pool_enter(const mcpi_space_s *sp)
 {
     ScratchPool &p = scratch();
     std::lock_guard<std::mutex> lock(p.mutex);
-    p.spaces[device] += step;
-    if (p.spaces[device] == 0 && p.pool[device]) cudaMemPoolTrimTo(p.pool[device], 0);
+    p.spaces[sp->device].push_back(sp);
 }
 
-// cudaMalloc, once more without the pool's unused memory when it fails for lack of it.
-template <class T>
-cudaError_t malloc_or_trim(int device, T **ptr, size_t bytes)
+void pool_leave(const mcpi_space_s *sp)
 {
-    cudaError_t e = cudaMalloc(ptr, bytes);
-    if (e != cudaErrorMemoryAllocation) return e;
-    (void)cudaGetLastError();
-    pool_trim(device);
-    return cudaMalloc(ptr, bytes);
+    ScratchPool &p = scratch();
+    std::lock_guard<std::mutex> lock(p.mutex);
+    auto &l = p.spaces[sp->device];
+    l.erase(std::remove(l.begin(), l.end(), sp), l.end());
+    if (l.empty() && p.pool[sp->device]) cudaMemPoolTrimTo(p.pool[sp->device], 0);
 }
 
 // The intermediate that the form of v passes between its halves: E (P x
@@ -377,11 +396,11 @@ int ensure_E(mcpi_space_s *sp, const PairOp &v)
     if (sp->N < 2) return MCPI_OK;
     const int form = mcpi::hpsi_form(sp->sp, v);
     if (form == mcpi::kFormContact) {
-        if (!sp->d_S && !mcpi::direct_covers(sp->sp)) CK(malloc_or_trim(sp->device, &sp->d_S, contact_bytes(sp)));
+        if (!sp->d_S && !mcpi::direct_covers(sp->sp)) CK(dev_malloc(sp, &sp->d_S, contact_bytes(sp)));
         return MCPI_OK;
     }
     if (form == mcpi::kFormDirect) return MCPI_OK;
-    if (!sp->d_E) CK(malloc_or_trim(sp->device, &sp->d_E, sizeof(double2) * (size_t)sp->P * sp->nc2));
+    if (!sp->d_E) CK(dev_malloc(sp, &sp->d_E, sizeof(double2) * (size_t)sp->P * sp->nc2));
     return ensure_fused(sp);
 }
 
@@ -430,7 +449,7 @@ int reserve(mcpi_space_s *sp, void *&ptr, size_t &cap, size_t bytes)
     cudaFree(ptr);
     ptr = nullptr;
     cap = 0;
-    CK(malloc_or_trim(sp->device, &ptr, bytes ? bytes : 1));
+    CK(dev_malloc(sp, &ptr, bytes ? bytes : 1));
     cap = bytes;
     return MCPI_OK;
 }
@@ -460,7 +479,7 @@ int ensure_fused(mcpi_space_s *sp)
     const size_t oc = ((size_t)nct + np + nct + 31) & ~size_t(31);
     const size_t words = oc + mcpi::kFusedCtlWords + ngroups;
     free_fused(sp);
-    CK(cudaMalloc(&sp->d_fz, sizeof(int) * words));
+    CK(dev_malloc(sp, &sp->d_fz, sizeof(int) * words));
     int *need = sp->d_fz, *order = need + nct;
     unsigned *ctl = (unsigned *)(sp->d_fz + oc), *count = ctl + mcpi::kFusedCtlWords;
     CK(cudaMemsetAsync(ctl, 0, sizeof(unsigned) * ((size_t)mcpi::kFusedCtlWords + ngroups), sp->stream));
@@ -533,7 +552,7 @@ int ensure_gram(mcpi_space_s *sp)
     if (sp->gram_cap >= need) return MCPI_OK;
     cudaFree(sp->d_gram);
     sp->d_gram = nullptr;
-    CK(malloc_or_trim(sp->device, &sp->d_gram, sizeof(double2) * need));
+    CK(dev_malloc(sp, &sp->d_gram, sizeof(double2) * need));
     sp->gram_cap = need;
     return MCPI_OK;
 }
@@ -560,6 +579,15 @@ extern "C" {
 static int check_status(mcpi_space_s *sp);
 
 }  // extern "C"
+
+cudaError_t mcpi::device_malloc(int device, void **ptr, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    (void)cudaGetLastError();
+    pool_trim(device);
+    return cudaMalloc(ptr, bytes);
+}
 
 int mcpi::set_error(int code, const char *msg)
 {
@@ -615,10 +643,10 @@ int mcpi_space_create(int N, int M, int device, mcpi_space *out)
     CHECK_ARG(device >= 0 && device < ndev && device < 64, "invalid device ordinal");
     DeviceGuard g(device);
     auto *s = new mcpi_space_s;
-    pool_space(device, 1);
     s->N = N;
     s->M = M;
     s->device = device;
+    pool_enter(s);
     s->nc = nc;
     s->nc1 = N >= 1 ? nc_exact(N - 1, M) : 0;
     s->nc2 = N >= 2 ? nc_exact(N - 2, M) : 0;
@@ -642,10 +670,10 @@ int mcpi_space_create(int N, int M, int device, mcpi_space *out)
     std::vector<double> sq(ws);
     for (int n = 0; n < ws; ++n) sq[n] = std::sqrt((double)n);
     cudaError_t e = cudaStreamCreateWithFlags(&s->own, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_W, sizeof(uint32_t) * W.size());
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_sq, sizeof(double) * ws);
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_dot, sizeof(double2) * (mcpi::lanczos_parts(nc) + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&s->d_status, sizeof(int));
+    if (e == cudaSuccess) e = dev_malloc(s, &s->d_W, sizeof(uint32_t) * W.size());
+    if (e == cudaSuccess) e = dev_malloc(s, &s->d_sq, sizeof(double) * ws);
+    if (e == cudaSuccess) e = dev_malloc(s, &s->d_dot, sizeof(double2) * (mcpi::lanczos_parts(nc) + 1));
+    if (e == cudaSuccess) e = dev_malloc(s, &s->d_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(s->d_status, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemcpy(s->d_W, W.data(), sizeof(uint32_t) * W.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(s->d_sq, sq.data(), sizeof(double) * ws, cudaMemcpyHostToDevice);
@@ -654,7 +682,7 @@ int mcpi_space_create(int N, int M, int device, mcpi_space *out)
         return fail(e == cudaErrorMemoryAllocation ? MCPI_ERR_NOMEM : MCPI_ERR_CUDA,
                     "mcpi_space_create: %s", cudaGetErrorString(e));
     }
-    s->stream = s->own;
+    mcpi_space_set_stream(s, s->own);
     *out = s;
     return MCPI_OK;
 }
@@ -687,8 +715,8 @@ static cudaError_t make_host_pipe(mcpi_space sp, size_t bytes)
     cudaError_t e = cudaStreamCreateWithFlags(&sp->s_h2d, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&sp->s_d2h, cudaStreamNonBlocking);
     for (int b = 0; b < 2 && e == cudaSuccess; ++b) {
-        e = cudaMalloc(&sp->d_hin[b], bytes);
-        if (e == cudaSuccess) e = cudaMalloc(&sp->d_hout[b], bytes);
+        e = dev_malloc(sp, &sp->d_hin[b], bytes);
+        if (e == cudaSuccess) e = dev_malloc(sp, &sp->d_hout[b], bytes);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sp->ev_in[b], cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sp->ev_comp[b], cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sp->ev_out[b], cudaEventDisableTiming);
@@ -706,6 +734,7 @@ int mcpi_space_destroy(mcpi_space sp)
     if (!sp) return MCPI_OK;
     DeviceGuard g(sp->device);
     if (sp->stream) cudaStreamSynchronize(sp->stream);
+    pool_leave(sp);
     free_op(sp->fwd);
     free_op(sp->adj);
     cudaFree(sp->d_W);
@@ -726,7 +755,6 @@ int mcpi_space_destroy(mcpi_space sp)
     free_fused(sp);
     cudaFree(sp->d_mr);
     if (sp->own) cudaStreamDestroy(sp->own);
-    pool_space(sp->device, -1);
     delete sp;
     return MCPI_OK;
 }
@@ -734,6 +762,7 @@ int mcpi_space_destroy(mcpi_space sp)
 int mcpi_space_set_stream(mcpi_space sp, void *stream)
 {
     CHECK_ARG(sp, "null space");
+    std::lock_guard<std::mutex> lock(scratch().mutex);   // pool_trim reads it from any thread
     sp->stream = (cudaStream_t)stream;   // NULL selects the legacy default stream
     return MCPI_OK;
 }
@@ -813,7 +842,7 @@ int mcpi_alloc(mcpi_space sp, size_t bytes, void **d_ptr)
     CHECK_ARG(sp && d_ptr, "null argument");
     DeviceGuard g(sp->device);
     *d_ptr = nullptr;
-    CK(cudaMalloc(d_ptr, bytes ? bytes : 1));
+    CK(dev_malloc(sp, d_ptr, bytes ? bytes : 1));
     return MCPI_OK;
 }
 
@@ -925,12 +954,12 @@ int mcpi_two_map_size(mcpi_space sp, int two_orbital, int64_t *entries)
     void *scratch = nullptr;
     size_t need = 0;
     int rc = MCPI_OK;
-    cudaError_t e = cudaMalloc(&cnt, sizeof(int64_t) * sp->nc);
-    if (e == cudaSuccess) e = cudaMalloc(&stride, sizeof(int64_t) * sp->nc);
-    if (e == cudaSuccess) e = cudaMalloc(&tot, sizeof(int64_t));
+    cudaError_t e = dev_malloc(sp, &cnt, sizeof(int64_t) * sp->nc);
+    if (e == cudaSuccess) e = dev_malloc(sp, &stride, sizeof(int64_t) * sp->nc);
+    if (e == cudaSuccess) e = dev_malloc(sp, &tot, sizeof(int64_t));
     if (e == cudaSuccess) e = mcpi::launch_chunk_counts(sp->sp, sp->tables(), two_orbital, cnt, sp->stream);
     if (e == cudaSuccess) e = mcpi::launch_stride_scan(sp->sp, cnt, stride, tot, nullptr, 0, &need, sp->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&scratch, need ? need : 1);
+    if (e == cudaSuccess) e = dev_malloc(sp, &scratch, need ? need : 1);
     if (e == cudaSuccess) e = mcpi::launch_stride_scan(sp->sp, cnt, stride, tot, scratch, need, nullptr, sp->stream);
     int64_t chunks = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&chunks, tot, sizeof(int64_t), cudaMemcpyDeviceToHost, sp->stream);
@@ -952,11 +981,11 @@ int mcpi_two_map(mcpi_space sp, int two_orbital, int64_t *d_stride, int32_t *d_m
     void *scratch = nullptr;
     size_t need = 0;
     int rc = MCPI_OK;
-    cudaError_t e = cudaMalloc(&cnt, sizeof(int64_t) * sp->nc);
-    if (e == cudaSuccess) e = cudaMalloc(&tot, sizeof(int64_t));
+    cudaError_t e = dev_malloc(sp, &cnt, sizeof(int64_t) * sp->nc);
+    if (e == cudaSuccess) e = dev_malloc(sp, &tot, sizeof(int64_t));
     if (e == cudaSuccess) e = mcpi::launch_chunk_counts(sp->sp, sp->tables(), two_orbital, cnt, sp->stream);
     if (e == cudaSuccess) e = mcpi::launch_stride_scan(sp->sp, cnt, d_stride, tot, nullptr, 0, &need, sp->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&scratch, need ? need : 1);
+    if (e == cudaSuccess) e = dev_malloc(sp, &scratch, need ? need : 1);
     if (e == cudaSuccess) e = mcpi::launch_stride_scan(sp->sp, cnt, d_stride, tot, scratch, need, nullptr, sp->stream);
     if (e == cudaSuccess) e = mcpi::launch_two_map(sp->sp, sp->tables(), two_orbital, d_stride, d_map, sp->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);
@@ -1002,7 +1031,7 @@ int mcpi_set_integrals(mcpi_space sp, const double *h_Ho, const double *h_Hint, 
     const int bits = mcpi::occ_bits_for(sp->N, sp->M);
     if (!sp->d_occ && !sp->no_occ && bits && sp->N >= 2 && sp->nc2 > 0) {
         const size_t b1 = sizeof(uint64_t) * (size_t)sp->nc, b2 = sizeof(uint64_t) * (size_t)sp->nc2;
-        if (cudaMalloc(&sp->d_occ, b1) == cudaSuccess && cudaMalloc(&sp->d_occ2, b2) == cudaSuccess) {
+        if (dev_malloc(sp, &sp->d_occ, b1) == cudaSuccess && dev_malloc(sp, &sp->d_occ2, b2) == cudaSuccess) {
             const mcpi::SpaceTables t{sp->d_W, sp->d_sq};
             mcpi::Space s2 = sp->sp;
             s2.N = sp->N - 2;
@@ -1039,15 +1068,7 @@ int mcpi_apply_h_host(mcpi_space sp, int count, const void *const *h_C, void *co
     int rc = ensure_E(sp, fop);
     if (rc) return rc;
     const size_t bytes = sizeof(double2) * (size_t)sp->nc;
-    if (!sp->host_pipe_ready) {
-        cudaError_t e = make_host_pipe(sp, bytes);
-        if (e == cudaErrorMemoryAllocation) {
-            (void)cudaGetLastError();
-            pool_trim(sp->device);
-            e = make_host_pipe(sp, bytes);
-        }
-        CK(e);
-    }
+    if (!sp->host_pipe_ready) CK(make_host_pipe(sp, bytes));
     fop = op_view(sp, sp->fwd);
     const HpsiScratch scratch(sp, fop);
     // buffer pair b = k & 1: its input is free once H.psi of state k-2 has run,
@@ -1148,7 +1169,7 @@ static int apply_rows(mcpi_space sp, const void *d_C, int64_t row0, int64_t row1
     uint32_t m0 = 0, m1 = 0xffffffffu;
     if (part && sp->fwd.hblk && sp->M >= 2 && mcpi::hpsi_form(sp->sp, fop) != mcpi::kFormDirect) {
         if (sp->mr_r0 != row0 || sp->mr_r1 != row1) {
-            if (!sp->d_mr) CK(cudaMalloc(&sp->d_mr, 2 * sizeof(uint32_t)));
+            if (!sp->d_mr) CK(dev_malloc(sp, &sp->d_mr, 2 * sizeof(uint32_t)));
             uint32_t h[2];
             CK(mcpi::launch_rows_mrange(sp->sp, sp->tables(), (uint32_t)row0, (uint32_t)row1, sp->d_mr, sp->stream));
             CK(cudaMemcpyAsync(h, sp->d_mr, sizeof h, cudaMemcpyDeviceToHost, sp->stream));
@@ -1192,7 +1213,7 @@ static int density(mcpi_space sp, int order, const void *phi, const void *psi, v
     // rho1 reads the packed occupations of the (N-1)-space, built on its first
     // call with the bits of the space's other tables (none: the kernel decodes)
     if (order == 1 && !sp->d_occ1 && sp->occ_bits && sp->nc1 > 0) {
-        if (cudaMalloc(&sp->d_occ1, sizeof(uint64_t) * (size_t)sp->nc1) == cudaSuccess) {
+        if (dev_malloc(sp, &sp->d_occ1, sizeof(uint64_t) * (size_t)sp->nc1) == cudaSuccess) {
             mcpi::Space s1 = sp->sp;
             s1.N = sp->N - 1;
             s1.nc = (uint32_t)sp->nc1;
@@ -1420,7 +1441,7 @@ int mcpi_ground(mcpi_space sp, void *d_C, int niter, double *E0, int *iters)
     if (mcpi::tridiag_lowest(n, d.data(), ee.data(), &Emin, zc.data()) != 0)
         return fail(MCPI_ERR_NUMERIC, "tridiagonal QL did not converge");
     double *dz = nullptr;
-    e = cudaMalloc(&dz, sizeof(double) * n);
+    e = dev_malloc(sp, &dz, sizeof(double) * n);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dz, zc.data(), sizeof(double) * n, cudaMemcpyHostToDevice, sp->stream);
     if (e == cudaSuccess) e = mcpi::launch_combine(V, n, nc, dz, (double2 *)d_C, sp->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);
@@ -1452,8 +1473,8 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
                           2 * sizeof(int);
     char *blk = nullptr;
     double2 *vec = nullptr;   // v[0], v[1], r, acc
-    CK(malloc_or_trim(sp->device, &blk, sbytes));
-    cudaError_t e = malloc_or_trim(sp->device, &vec, sizeof(double2) * nc * 4);
+    CK(dev_malloc(sp, &blk, sbytes));
+    cudaError_t e = dev_malloc(sp, &vec, sizeof(double2) * nc * 4);
     if (e != cudaSuccess) {
         cudaFree(blk);
         return fail(MCPI_ERR_NOMEM, "mcpi_ground_lowmem: %s", cudaGetErrorString(e));

@@ -38,6 +38,10 @@ struct DevPairOp {
     BlockOp blocks() const { return BlockOp{prog, prog_bytes}; }
 };
 
+// cudaMalloc on the current device `device`; when memory is short, once more after
+// the unused memory of the library's scratch pool has gone back to the device.
+cudaError_t device_malloc(int device, void **ptr, size_t bytes);
+
 // Records msg as the calling thread's mcpi_last_error() and returns code.
 int set_error(int code, const char *msg);
 

@@ -143,6 +143,18 @@ API cudaError_t cudaMemPoolCreate(cudaMemPool_t *p, const cudaMemPoolProps *)
     return cudaSuccess;
 }
 API cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
+API cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, cudaMemPoolAttr a, void *v)
+{
+    if (a != cudaMemPoolAttrReservedMemCurrent) return ret(cudaErrorInvalidValue);
+    *static_cast<uint64_t *>(v) = f().pool_reserved;
+    return cudaSuccess;
+}
+API cudaError_t cudaMemGetInfo(size_t *free, size_t *total)
+{
+    *free = left();
+    *total = f().capacity;
+    return cudaSuccess;
+}
 API cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t)
 {
     for (auto &b : f().pool_ready) {

@@ -1,10 +1,12 @@
 """Host code of the library without a GPU (tests/fake_cuda.py): a launch that
 fails fails the call it belongs to."""
+import ctypes as ct
+
 import pytest
 
 import fake_cuda
 import mcpi_b200 as mc
-from fake_cuda import ERR_CUDA, OK
+from fake_cuda import ERR_CUDA, ERR_NOMEM, OK
 
 
 @pytest.fixture(scope="session")
@@ -160,3 +162,93 @@ def test_solve_rows_is_per_thread_and_nests():
             pass
         seen.append(_rows.solve)
     assert seen == [True, False, True] and not _rows.solve
+
+
+class Held:
+    """A space of 13 bosons in 10 orbitals with one H.psi queued: the pool holds
+    its S, 51 MB, freed on the stream but not seen to be. On the device then no
+    more than `room` bytes are left beside it."""
+
+    def __init__(self, fake, room):
+        self.s = fake.space(13, 10)
+        assert self.s.set_integrals(*mc.lieb_integrals(10, 1.0)) == OK
+        self.fake, self.room = fake, room
+
+    def __enter__(self):
+        assert forms(self.fake.kernels(self.s.apply_h)) == {"contact"}
+        assert self.fake.L.fake_pool_held() > 50e6
+        self.fake.L.fake_headroom(self.room)
+        return self
+
+    def __exit__(self, *exc):
+        self.fake.reset()
+        self.s.close()
+
+
+def alloc(s, n):
+    p = ct.c_void_p()
+    rc = s.L.mcpi_alloc(s.h, ct.c_size_t(n), ct.byref(p))
+    if rc == OK:
+        s.L.mcpi_free(s.h, p)
+    return rc
+
+
+def packs(kernels):
+    return len([n for n in kernels if "k_pack_occ" in n])
+
+
+def test_pool_memory_goes_to_an_allocation(fake):
+    with Held(fake, 1 << 20) as h:
+        assert alloc(h.s, 40 << 20) == OK and fake.L.fake_pool_held() == 0
+        assert alloc(h.s, 80 << 20) == ERR_NOMEM              # more than there is stays refused
+        assert forms(fake.kernels(h.s.apply_h)) == {"contact"}
+
+
+def test_pool_memory_goes_to_the_tables(fake):
+    t = fake.space(11, 11)                                     # occupations 2.8 and 0.7 MB, rho1's 1.5 MB
+    with Held(fake, 1 << 20):
+        assert packs(fake.kernels(lambda: t.set_integrals(*mc.lieb_integrals(11, 1.0)))) == 2
+    assert t.density(2) == OK                                  # the partial sums, not counted here
+    with Held(fake, 1 << 20):
+        assert packs(fake.kernels(lambda: t.density(1))) == 1
+    n = ct.c_int64()
+    with Held(fake, 1 << 20):
+        assert t.L.mcpi_two_map_size(t.h, 1, ct.byref(n)) == OK
+    t.close()
+
+
+def test_pool_memory_goes_to_an_operator_and_a_space(fake):
+    _, Ho, Hint = mc.random_problem(4, 12, 3)
+    t = fake.space(4, 12)                                      # dense pair matrices, 97 kB each
+    with Held(fake, 40 << 10):
+        assert t.set_integrals(Ho, Hint) == OK
+    t.close()
+    with Held(fake, 64):
+        u = fake.space(4, 4)
+        u.close()
+
+
+def test_pool_memory_goes_to_a_batch(fake):
+    # arena 36 MB with the contact form's intermediates, 21 MB without
+    members = [(10, 10), (10, 10)]
+    with Held(fake, 30 << 20):
+        b = fake.batch(members, 5, mc.lieb_integrals)
+        assert b.rc == OK and any("k_batch_contact" in n for n in fake.kernels(b.run))
+        b.close()
+
+
+def test_a_batch_leaves_room_for_its_tables(fake):
+    # With room for the larger arena but not for what the batch still needs
+    # after it, the batch takes the smaller arena and runs the direct form.
+    members, later = [(10, 10), (10, 10)], 2 * ((1 << 20) + 8 * (92378 + 24310))
+    b = fake.batch(members, 5, mc.lieb_integrals)
+    n = ct.c_size_t()
+    b.L.mcpi_batch_arena_bytes(b.h, ct.byref(n))
+    b.close()
+    for room, contact in ((n.value + later + (1 << 20), True), (n.value + (1 << 16), False)):
+        fake.L.fake_headroom(room)
+        b = fake.batch(members, 5, mc.lieb_integrals)
+        assert b.rc == OK
+        assert any("k_batch_contact" in k for k in fake.kernels(b.run)) == contact
+        b.close()
+        fake.reset()
