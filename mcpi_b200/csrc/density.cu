@@ -604,13 +604,13 @@ __device__ __forceinline__ void rho1_part(const Space &sp, const SpaceTables &tb
 #pragma unroll
         for (int l = B0; l < B1; ++l) {
             y[l - B0] = __ldg(psi + (base + d[l]));
-            fy[l - B0] = in ? sq[u[l] + 1] : 0.0;
+            fy[l - B0] = sq[u[l] + 1];
         }
         if constexpr (!SAME) {
 #pragma unroll
             for (int l = A0; l < A1; ++l) {
                 z[l - A0] = __ldg(phi + (base + d[l]));
-                fz[l - A0] = in ? sq[u[l] + 1] : 0.0;
+                fz[l - A0] = sq[u[l] + 1];
             }
         }
     };
@@ -624,6 +624,15 @@ __device__ __forceinline__ void rho1_part(const Space &sp, const SpaceTables &tb
         if constexpr (!SAME) {
 #pragma unroll
             for (int l = 0; l < NZ; ++l) q[l] = make_double2(fz[l] * z[l].x, fz[l] * z[l].y);
+        }
+        // lanes past the last configuration hold the first one's values, which may be
+        // infinite: they add zeros, not zero times those (predicated loads instead
+        // made rho1 at N=20, M=10 289 -> 318 us)
+        if (tile + 1 == ntiles && tile * 32 + lane >= nh) {
+#pragma unroll
+            for (int l = 0; l < B1 - B0; ++l) p[l] = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int l = 0; l < NZ; ++l) q[l] = make_double2(0.0, 0.0);
         }
         if (R::AHEAD && tile + step < ntiles) fetch(tile + step);
         int e = -E0;
