@@ -1418,6 +1418,12 @@ int mcpi_tridiag_eig(int n, double *d, double *e, double *z)
     return MCPI_OK;
 }
 
+static int tridiag_failed(int t)
+{
+    return t == -2 ? fail(MCPI_ERR_NOMEM, "no host memory for the tridiagonal eigenproblem")
+                   : fail(MCPI_ERR_NUMERIC, "tridiagonal QL did not converge");
+}
+
 int mcpi_ground(mcpi_space sp, void *d_C, int niter, double *E0, int *iters)
 {
     CHECK_ARG(sp && d_C && E0 && niter >= 1, "mcpi_ground: bad arguments");
@@ -1438,8 +1444,7 @@ int mcpi_ground(mcpi_space sp, void *d_C, int niter, double *E0, int *iters)
     for (int k = 0; k < n; ++k) d[k] = diag[2 * k];
     for (int k = 0; k + 1 < n; ++k) ee[k] = off[k];
     double Emin = 0.0;
-    if (mcpi::tridiag_lowest(n, d.data(), ee.data(), &Emin, zc.data()) != 0)
-        return fail(MCPI_ERR_NUMERIC, "tridiagonal QL did not converge");
+    if (const int t = mcpi::tridiag_lowest(n, d.data(), ee.data(), &Emin, zc.data())) return tridiag_failed(t);
     double *dz = nullptr;
     e = dev_malloc(sp, &dz, sizeof(double) * n);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dz, zc.data(), sizeof(double) * n, cudaMemcpyHostToDevice, sp->stream);
@@ -1521,10 +1526,10 @@ int mcpi_ground_lowmem(mcpi_space sp, void *d_C, int niter, double *E0, int *ite
     if (e == cudaSuccess) {
         for (int k = 0; k < n; ++k) d[k] = alpha[k].x;
         for (int k = 0; k + 1 < n; ++k) ee[k] = beta[k];
-        if (mcpi::tridiag_lowest(n, d.data(), ee.data(), &Emin, zc.data()) != 0) {
+        if (const int t = mcpi::tridiag_lowest(n, d.data(), ee.data(), &Emin, zc.data())) {
             cudaFree(blk);
             cudaFree(vec);
-            return fail(MCPI_ERR_NUMERIC, "tridiagonal QL did not converge");
+            return tridiag_failed(t);
         }
     }
     // pass 2: regenerate v_0 .. v_{n-1} and accumulate sum_k z_k v_k
