@@ -76,14 +76,16 @@ MCPI_API int mcpi_space_sync(mcpi_space sp);
  * otherwise chosen for M <= 12). Takes effect at the next mcpi_set_integrals. */
 #define MCPI_OPT_NO_GEMM_KERNEL 4
 /* MCPI_OPT_WAIT_LIMIT_KCYCLES (>= 0): limit, in thousands of SM cycles, of
- * each bounded wait inside the warp-specialised dense-product kernel (0, the
- * default: about two seconds). A wait that runs out makes the kernel return
+ * each bounded wait inside a kernel: the dense product and the tensor-core Gram,
+ * the fused H.psi, the one-launch Lanczos (0, the default: about two seconds). A
+ * wait that runs out makes the kernel return
  * and the next synchronising call report MCPI_ERR_TIMEOUT. */
 #define MCPI_OPT_WAIT_LIMIT_KCYCLES 5
 /* MCPI_OPT_TEST_STALL_GATHER (0/1): for testing the timeout paths only — the
  * gather warps of the dense-product and tensor-core Gram kernels deliver no
- * tile and the fused H.psi kernel's producers never count themselves done, so
- * the waits run out (results are invalid while it is set). */
+ * tile, the fused H.psi kernel's producers never count themselves done and one
+ * block of the one-launch Lanczos never arrives at its barriers, so the waits run
+ * out (results are invalid while it is set). */
 #define MCPI_OPT_TEST_STALL_GATHER 6
 /* MCPI_OPT_NO_OCC_TABLES (0/1): build no packed occupation tables (the H.psi
  * kernels then decode every row index; 1 also frees existing tables). Takes

@@ -186,6 +186,7 @@ struct SmallArgs {
     unsigned *ctl;            // barrier counter, abort flag (zero at launch)
     int *status;
     long long wait_cycles;
+    int test_stall;           // block 0 never arrives, so that the waits run out
 };
 
 // Grid barrier number k (0, 1, ..): false once any block has given up.
@@ -259,6 +260,7 @@ __global__ void __launch_bounds__(kST, 1) k_small_lanczos(SmallArgs a)
     const RowLists &rl = a.rl;
     unsigned nbar = 0;
     double beta = 0.0, maxbeta = 0.0;
+    if (a.test_stall && blockIdx.x == 0) return;
     for (int i = -1; i < a.lm - 1; ++i) {
         // this step makes v_{i+1} (i = -1: v_0 is given), alpha_{i+1} and the next residual
         double2 *vn = a.V + (size_t)(i + 1) * nc;
@@ -521,6 +523,7 @@ cudaError_t launch_small_lanczos(const Space &sp, const SpaceTables &tb, const P
     a.ctl = reinterpret_cast<unsigned *>(b + lay.ctl);
     a.status = op.status;
     a.wait_cycles = op.wait_cycles;
+    a.test_stall = op.test_stall;
     int sms = 0, per = 0;
     const size_t sm = small_smem(sp, lm);
     const void *fn = (const void *)k_small_lanczos;
