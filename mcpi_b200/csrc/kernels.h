@@ -297,8 +297,6 @@ cudaError_t launch_dot(const double2 *a, const double2 *b, int64_t nc, double2 *
 // the launch sequence leaves them (s.iters preset to lm), work of
 // small_lanczos_bytes. cudaErrorCooperativeLaunchTooLarge: cannot run here,
 // nothing was enqueued.
-constexpr uint32_t kSmallMaxRows = 16384;
-constexpr int kSmallMinSteps = 8;
 bool small_lanczos_fits(const Space &sp, int lm);
 size_t small_lanczos_bytes(const Space &sp, int lm);
 cudaError_t launch_small_lanczos(const Space &sp, const SpaceTables &tb, const PairOp &op, double2 *V, int lm,

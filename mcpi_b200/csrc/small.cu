@@ -482,14 +482,30 @@ struct SmallLayout {
     }
 };
 
-constexpr size_t kSmallSmem = 226 * 1024;   // of the 227 KB a block may have (the rest: static)
+// The solves that it takes: up to this many rows (every block keeps the whole
+// vector in shared memory and reads it twice a step, which grows with the rows
+// while the launch sequence's short kernels do not), and enough steps to pay for
+// the lists, one per 128 rows. mcpi_ground in ms, one launch / launch sequence:
+//   N=18, M=4 (1,330 rows) 8 steps 0.20 / 0.28, 500 steps 17.6 / 25.2;
+//   N=5, M=11 (3,003) 40 steps 0.87 / 1.23, 500 steps 19.1 / 29.0;
+//   N=10, M=6 (3,003) 8 steps 0.239 / 0.232, 40 steps 0.85 / 0.99;
+//   N=9, M=7 (5,005) 8 steps 0.264 / 0.244, 40 steps 1.01 / 1.05, 500 steps 23.6 / 26.7;
+//   N=12, M=6 (6,188) 100 steps 2.78 / 2.70, 500 steps 24.6 / 26.2;
+//   N=14, M=6 (11,628) 100 steps 3.90 / 2.69.
+constexpr uint32_t kSmallMaxRows = 5500;
+constexpr int kSmallMinSteps = 8, kSmallMaxSteps = 2048;
+constexpr uint32_t kSmallRowsPerStep = 128;
+// Its shared memory never exceeds that of the largest such solve (66 pairs: M = 11).
+constexpr size_t kSmallSmem = sizeof(double2) * (kSmallMaxRows + kSmallMaxSteps + 32 * 66);
+static_assert(kSmallSmem <= 226 * 1024 && kDirectAutoMaxM * (kDirectAutoMaxM + 1) / 2 == 66 && kChunk <= 66,
+              "a block may have 227 KB, 1 KB of it static");
 
 }  // namespace
 
 bool small_lanczos_fits(const Space &sp, int lm)
 {
     return sp.M >= 2 && sp.N >= 2 && direct_covers(sp) && sp.nc <= kSmallMaxRows && lm >= kSmallMinSteps &&
-           lm <= 2048 && small_smem(sp, lm) <= kSmallSmem;
+           lm <= kSmallMaxSteps && kSmallRowsPerStep * (uint32_t)lm >= sp.nc;
 }
 
 size_t small_lanczos_bytes(const Space &sp, int lm) { return SmallLayout(sp, lm).bytes; }

@@ -252,3 +252,13 @@ def test_a_batch_leaves_room_for_its_tables(fake):
         assert any("k_batch_contact" in k for k in fake.kernels(b.run)) == contact
         b.close()
         fake.reset()
+
+
+@pytest.mark.parametrize("N,M,lm,one", [(2, 2, 7, False), (2, 2, 8, True), (5, 11, 23, False), (5, 11, 24, True),
+                                        (9, 7, 39, False), (9, 7, 40, True), (12, 6, 400, False), (6, 11, 400, False),
+                                        (9, 7, 2048, True), (2, 2, 2049, False)])
+def test_which_solves_take_one_launch(fake, N, M, lm, one):
+    s = fake.space(N, M)                   # 3, 3,003, 5,005, 6,188 and 8,008 rows
+    assert s.set_integrals(*mc.lieb_integrals(M, 1.0)) == OK
+    assert any("k_small_lanczos" in k for k in fake.kernels(lambda: s.lanczos(lm))) == one
+    s.close()
