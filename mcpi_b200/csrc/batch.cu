@@ -7,10 +7,10 @@
 // reorthogonalisation, breakdown at beta_i / max beta < 1e-15) but each
 // stage is one launch over all members:
 //   * H.psi: per orbital count M the contact form's two launches (M >= 10,
-//     contact interactions), one launch of the direct kernel (M <= 11, no
-//     intermediate) or one annihilation + one creation launch through the
-//     members' E (hpsi.cu, k_batch_*), blocks assigned from (member, block)
-//     work tables;
+//     contact interactions, where they pay: contact_group), one launch of the
+//     direct kernel (M <= 11, no intermediate) or one annihilation + one
+//     creation launch through the members' E (hpsi.cu, k_batch_*), blocks
+//     assigned from (member, block) work tables;
 //   * vector stages: blocks assigned from (member, 2048-row tile) work tables,
 //     per-member partial sums reduced in a fixed order by one block per member;
 //   * a member whose Lanczos broke down sets its flag and every later block of
@@ -382,6 +382,25 @@ namespace {
 
 int bfail(int code, const std::string &msg) { return mcpi::set_error(code, msg.c_str()); }
 
+// Whether a group of n members of M orbitals, `rows` rows together, takes the
+// contact form where its integrals allow it. Up to eleven orbitals it stands
+// against one launch of the direct kernel per batch_chunk_members(M) members, so
+// it pays where it needs no more launches than that, and otherwise from a size on
+// where the kernels' time counts more than a launch. 60 steps of a batch, contact
+// / direct in ms: M=10, 91,520 rows 3.56 / 3.52, 137,280 rows 4.48 / 4.53, 32,032
+// rows 3.25 / 2.96, 20 members and 14,300 rows 3.25 / 3.43; M=11, 64,064 rows 3.49
+// / 3.39, 96,096 rows 3.85 / 3.82, 36,036 rows 3.35 / 3.12; N=12, M=10 x 16, 40
+// steps 45.6 / 51.0. Above that it stands against the two pair kernels: M=12, 728
+// rows 3.02 / 3.36, M=16, 6,528 rows 3.87 / 4.59.
+bool contact_group(int M, int n, int64_t rows)
+{
+    if (M < mcpi::kBatchContactMinM) return false;
+    if (M > mcpi::kBatchDirectMaxM) return true;
+    const int c = mcpi::batch_contact_members(M), d = mcpi::batch_chunk_members(M);
+    if (2 * ((n + c - 1) / c) <= (n + d - 1) / d) return true;
+    return rows >= (M == 10 ? 128 * 1024 : 96 * 1024);
+}
+
 }  // namespace
 
 extern "C" {
@@ -421,6 +440,17 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
         b->lz[m].nc = nc;
         b->lz[m].ntiles = ntiles;
     }
+    bool contact[mcpi::kMaxM + 1] = {};   // per M
+    for (int x = 2; x <= mcpi::kMaxM; ++x) {
+        int n = 0;
+        int64_t rows = 0;
+        for (int m = 0; m < count; ++m)
+            if (M[m] == x) {
+                ++n;
+                rows += b->spaces[m]->nc;
+            }
+        contact[x] = contact_group(x, n, rows);
+    }
     // the arena, with the contact form's intermediate for members that the
     // direct form covers too as long as there is memory for it
     for (int with_S = 1; with_S >= 0 && !b->arena; --with_S) {
@@ -435,7 +465,7 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
             off_E[m] = tot;
             if (M[m] > mcpi::kBatchDirectMaxM)   // the two-kernel form's intermediate (the contact form's fits in it)
                 tot += mcpi::up256(sizeof(double2) * (size_t)s->P * s->nc2);
-            else if (with_S && M[m] >= mcpi::kBatchContactMinM)
+            else if (with_S && contact[M[m]])
                 tot += mcpi::up256(sizeof(double2) * (size_t)(2 * M[m] - 1) * s->nc2);
             off_S[m] = tot;
             tot += mcpi::up256(sizeof(double2) * nc);
@@ -481,7 +511,7 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
         bm.nh = 0;
         bm.hdiag = nullptr;
         bm.lvec = z.V;
-        bm.E = M[m] > mcpi::kBatchDirectMaxM || (b->has_S && M[m] >= mcpi::kBatchContactMinM)
+        bm.E = M[m] > mcpi::kBatchDirectMaxM || (b->has_S && contact[M[m]])
                    ? reinterpret_cast<double2 *>(b->arena + off_E[m])
                    : nullptr;
         bm.r = z.r;
@@ -546,7 +576,7 @@ int mcpi_batch_create(int count, const int *N, const int *M, int lm, int device,
     std::vector<std::vector<std::vector<int>>> pmem(Ms.size());
     std::vector<std::vector<std::vector<int2>>> pw1(Ms.size()), pw2(Ms.size());
     for (size_t g = 0; g < Ms.size(); ++g) {
-        if (Ms[g] < mcpi::kBatchContactMinM || !(b->has_S || Ms[g] > mcpi::kBatchDirectMaxM)) continue;
+        if (!contact[Ms[g]] || !(b->has_S || Ms[g] > mcpi::kBatchDirectMaxM)) continue;
         const int cap = mcpi::batch_contact_members(Ms[g]);
         for (int m = 0; m < count; ++m) {
             if (M[m] != Ms[g]) continue;

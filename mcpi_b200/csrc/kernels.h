@@ -221,8 +221,8 @@ size_t batch_contact_bytes(int M);
 void batch_fill_contact(int M, void *vals, int slot, int member, const double *uw);
 cudaError_t launch_batch_contact(int M, const BatchMember *mem, const int2 *work1, int n1, const int2 *work2, int n2,
                                  size_t smem1, size_t smem2, int vec, const void *vals, cudaStream_t st);
-// Orbital counts from which a batch takes the contact form where it can (its
-// members share the launches, so their sizes do not matter as in contact_pays).
+// Orbital counts from which a batch takes the contact form where it can and where
+// that pays (batch.cu: contact_group).
 constexpr int kBatchContactMinM = 10;
 // Sets the kernels' shared-memory limits (call outside stream capture).
 cudaError_t batch_prepare(int M, size_t smem1, size_t smem2, size_t smem3);

@@ -262,3 +262,15 @@ def test_which_solves_take_one_launch(fake, N, M, lm, one):
     assert s.set_integrals(*mc.lieb_integrals(M, 1.0)) == OK
     assert any("k_small_lanczos" in k for k in fake.kernels(lambda: s.lanczos(lm))) == one
     s.close()
+
+
+# 92,378 and 48,620 rows at M = 10, 92,378 and 43,758 at M = 11, 1,365 at M = 12
+@pytest.mark.parametrize("members,contact", [
+    ([(10, 10)], False), ([(10, 10), (9, 10)], True), ([(4, 10)] * 19, False), ([(4, 10)] * 20, True),
+    ([(9, 11)], False), ([(9, 11), (5, 11), (5, 11)], True), ([(3, 11)] * 14, False), ([(3, 11)] * 15, True),
+    ([(4, 12)], True), ([(10, 9)] * 3, False)])
+def test_which_batches_take_the_contact_form(fake, members, contact):
+    b = fake.batch(members, 4, mc.lieb_integrals)
+    assert b.rc == OK
+    assert any("k_batch_contact" in k for k in fake.kernels(b.run)) == contact
+    b.close()
