@@ -1861,8 +1861,9 @@ cudaError_t batch_prepare_m(size_t smem1, size_t smem2, size_t smem3)
         e = cudaFuncSetAttribute(k_batch_direct<M, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k_batch_direct_p<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_batch_contact_create<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    if constexpr (M >= kBatchContactMinM)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_batch_contact_create<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
     return e;
 }
 
@@ -1902,8 +1903,11 @@ cudaError_t apply_h_m(const Space &sp, const SpaceTables &tb, const PairOp &op, 
     const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
     if constexpr (M >= 2) {
         const int form = hpsi_form(sp, op);
-        if (form == kFormContact)
-            return contact_apply_m<M>(sp, tb, op, psi, E, out, stages, st, row0, row1, m0, m1);
+        // nine orbitals never take it: the direct form is faster up to N = 63
+        // (contact_pays), and N = 64 does not fit the configuration index
+        if constexpr (M != 9)
+            if (form == kFormContact)
+                return contact_apply_m<M>(sp, tb, op, psi, E, out, stages, st, row0, row1, m0, m1);
         if (stages == 3) {
             if (form == kFormDirect) return direct_apply_m<M>(sp, tb, op, psi, out, st, row0, row1);
             if (form == kFormFused && row0 == 0 && row1 == sp.nc)
@@ -2097,14 +2101,14 @@ cudaError_t launch_batch_direct_vals(int M, const BatchMember *mem, const int2 *
     }
 }
 
+// (groups take the contact form from kBatchContactMinM orbitals on)
+static_assert(kBatchContactMinM == 10, "the cases below");
 int batch_contact_members(int M)
 {
     switch (M) {
 #define MCPI_CASE(m) \
     case m: return BatchContact<m>::CAP;
-        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
-        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
-        MCPI_CASE(15) MCPI_CASE(16)
+        MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14) MCPI_CASE(15) MCPI_CASE(16)
 #undef MCPI_CASE
     default: return 0;
     }
@@ -2115,9 +2119,7 @@ size_t batch_contact_bytes(int M)
     switch (M) {
 #define MCPI_CASE(m) \
     case m: return sizeof(BatchContact<m>);
-        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
-        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
-        MCPI_CASE(15) MCPI_CASE(16)
+        MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14) MCPI_CASE(15) MCPI_CASE(16)
 #undef MCPI_CASE
     default: return 0;
     }
@@ -2151,9 +2153,7 @@ void batch_fill_contact(int M, void *vals, int slot, int member, const double *u
     switch (M) {
 #define MCPI_CASE(m) \
     case m: fill_contact_m<m>(vals, slot, member, uw); break;
-        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
-        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
-        MCPI_CASE(15) MCPI_CASE(16)
+        MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14) MCPI_CASE(15) MCPI_CASE(16)
 #undef MCPI_CASE
     default: break;
     }
@@ -2165,9 +2165,7 @@ cudaError_t launch_batch_contact(int M, const BatchMember *mem, const int2 *work
     switch (M) {
 #define MCPI_CASE(m) \
     case m: return launch_contact_m<m>(mem, work1, n1, work2, n2, smem1, smem2, vec, vals, st);
-        MCPI_CASE(2) MCPI_CASE(3) MCPI_CASE(4) MCPI_CASE(5) MCPI_CASE(6) MCPI_CASE(7) MCPI_CASE(8)
-        MCPI_CASE(9) MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14)
-        MCPI_CASE(15) MCPI_CASE(16)
+        MCPI_CASE(10) MCPI_CASE(11) MCPI_CASE(12) MCPI_CASE(13) MCPI_CASE(14) MCPI_CASE(15) MCPI_CASE(16)
 #undef MCPI_CASE
     default: return cudaErrorInvalidValue;
     }
