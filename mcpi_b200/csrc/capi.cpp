@@ -204,8 +204,8 @@ std::vector<cplx> pack_momentum(const std::vector<cplx> &Ht, int P, int M)
 // Outer-product factors of a momentum-block pair matrix (layout in kernels.h,
 // PairOp::contact): u[P] | w[P] with Ht[a][b] = u_a w_b inside every block,
 // all real. Each block's row and column through its largest entry give the
-// factors; empty when some value is complex or differs from its product by
-// more than rounding (4 ulp: the same values up to the order of multiplication).
+// factors; empty when some value is complex or is not exactly its product (the
+// kernels apply the product, and the operator is what the caller gave).
 std::vector<double> pack_contact(const std::vector<cplx> &Ht, int P, int M)
 {
     std::vector<double> f(2 * (size_t)P, 0.0);
@@ -227,7 +227,7 @@ std::vector<double> pack_contact(const std::vector<cplx> &Ht, int P, int M)
         for (int r = 0; r < n; ++r)
             for (int c = 0; c < n; ++c) {
                 const double h = at(r, c).real();
-                if (!(std::fabs(f[pr(r)] * f[(size_t)P + pr(c)] - h) <= 8.9e-16 * std::fabs(h))) return {};
+                if (f[pr(r)] * f[(size_t)P + pr(c)] != h) return {};
             }
     }
     return f;

@@ -2,6 +2,7 @@
 fails fails the call it belongs to."""
 import ctypes as ct
 
+import numpy as np
 import pytest
 
 import fake_cuda
@@ -274,3 +275,20 @@ def test_which_batches_take_the_contact_form(fake, members, contact):
     assert b.rc == OK
     assert any("k_batch_contact" in k for k in fake.kernels(b.run)) == contact
     b.close()
+
+
+def scaled_contact(M, g, f):
+    """Contact integrals with a real factor per orbital."""
+    Ho, Hint = mc.lieb_integrals(M, g)
+    return Ho, (Hint.reshape(M, M, M, M) * np.einsum("l,q,s,k->lqsk", f, f, f, f)).reshape(-1)
+
+
+def test_the_contact_form_takes_exact_products_only(fake):
+    M = 12
+    for f, exact in ((np.ones(M), True), (2.0 ** np.arange(-6, 6), True), (-np.ones(M), True),
+                     (np.random.default_rng(1).uniform(0.5, 2.0, M), False)):
+        s = fake.space(4, M)
+        assert s.set_integrals(*scaled_contact(M, 0.7, f)) == OK
+        assert forms(fake.kernels(s.apply_h)) == {"contact" if exact else "pairs"}
+        assert forms(fake.kernels(s.apply_h_adjoint)) == {"contact" if exact else "pairs"}
+        s.close()
