@@ -1038,7 +1038,9 @@ int mcpi_set_integrals(mcpi_space sp, const double *h_Ho, const double *h_Hint, 
             s2.nc = (uint32_t)sp->nc2;
             cudaError_t e = mcpi::launch_pack_occ(sp->sp, t, sp->d_occ, bits, sp->stream);
             if (e == cudaSuccess) e = mcpi::launch_pack_occ(s2, t, sp->d_occ2, bits, sp->stream);
-            if (e != cudaSuccess) {   // no table is left that was not written
+            // written before any stream can read them, the space's next one included
+            if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);
+            if (e != cudaSuccess) {   // no table is left that may not have been written
                 cudaFree(sp->d_occ);
                 cudaFree(sp->d_occ2);
                 sp->d_occ = sp->d_occ2 = nullptr;
@@ -1211,14 +1213,18 @@ static int density(mcpi_space sp, int order, const void *phi, const void *psi, v
     int rc = ensure_gram(sp);
     if (rc) return rc;
     // rho1 reads the packed occupations of the (N-1)-space, built on its first
-    // call with the bits of the space's other tables (none: the kernel decodes)
-    if (order == 1 && !sp->d_occ1 && sp->occ_bits && sp->nc1 > 0) {
+    // call with the bits of the space's other tables (none: the kernel decodes), and
+    // not under capture, where they would be written by a replay only
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (order == 1 && !sp->d_occ1 && sp->occ_bits && sp->nc1 > 0 &&
+        cudaStreamIsCapturing(sp->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
         if (dev_malloc(sp, &sp->d_occ1, sizeof(uint64_t) * (size_t)sp->nc1) == cudaSuccess) {
             mcpi::Space s1 = sp->sp;
             s1.N = sp->N - 1;
             s1.nc = (uint32_t)sp->nc1;
-            const cudaError_t e = mcpi::launch_pack_occ(s1, mcpi::SpaceTables{sp->d_W, sp->d_sq}, sp->d_occ1,
-                                                        sp->occ_bits, sp->stream);
+            cudaError_t e = mcpi::launch_pack_occ(s1, mcpi::SpaceTables{sp->d_W, sp->d_sq}, sp->d_occ1, sp->occ_bits,
+                                                  sp->stream);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);   // as above
             if (e != cudaSuccess) {
                 cudaFree(sp->d_occ1);
                 sp->d_occ1 = nullptr;

@@ -30,6 +30,7 @@ struct Fake {
     std::map<void *, size_t> blocks, pool_live, pool_pending, pool_ready;
     size_t pool_reserved = 0;
     int capturing = 0;
+    size_t synced_log = 0;               // length of the log at the last synchronisation
     int optin = 232448;                  // shared memory a block may opt in to
     cudaError_t last = cudaSuccess;
 };
@@ -60,6 +61,7 @@ size_t left()
 
 void synced()
 {
+    f().synced_log = f().log.size();
     for (auto &b : f().pool_pending) f().pool_ready.insert(b);
     f().pool_pending.clear();
 }
@@ -103,7 +105,13 @@ API void fake_reset()
     f().last = cudaSuccess;
 }
 API const char *fake_log() { return f().log.c_str(); }
-API void fake_clear_log() { f().log.clear(); }
+API void fake_clear_log()
+{
+    f().log.clear();
+    f().synced_log = 0;
+}
+API size_t fake_synced_log() { return f().synced_log; }
+API void fake_capture(int on) { f().capturing = on; }
 API void fake_fail_launch(long k) { f().fail_launch = k; }
 API void fake_fail_pool(long k, int all)
 {

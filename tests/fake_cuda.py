@@ -31,8 +31,9 @@ class Fake:
         self.L = L = ct.CDLL(so)
         L.fake_log.restype = ct.c_char_p
         L.mcpi_last_error.restype = ct.c_char_p
-        for f in ("fake_headroom", "fake_pool_held", "fake_used"):
+        for f in ("fake_pool_held", "fake_used", "fake_synced_log"):
             getattr(L, f).restype = ct.c_size_t
+        L.fake_headroom.restype = None
         L.fake_headroom.argtypes = [ct.c_size_t]
         L.fake_fail_launch.argtypes = [ct.c_long]
         L.fake_fail_pool.argtypes = [ct.c_long, ct.c_int]
@@ -45,6 +46,12 @@ class Fake:
         self.L.fake_clear_log()
         assert call() == OK, self.L.mcpi_last_error()
         return self.L.fake_log().decode().split()
+
+    def unfinished(self, call):
+        """Names of the kernels launched by call() that the host has not waited for at its end."""
+        self.L.fake_clear_log()
+        assert call() == OK, self.L.mcpi_last_error()
+        return self.L.fake_log()[self.L.fake_synced_log():].decode().split()
 
     def space(self, N, M):
         return Space(self, N, M)

@@ -292,3 +292,18 @@ def test_the_contact_form_takes_exact_products_only(fake):
         assert forms(fake.kernels(s.apply_h)) == {"contact" if exact else "pairs"}
         assert forms(fake.kernels(s.apply_h_adjoint)) == {"contact" if exact else "pairs"}
         s.close()
+
+
+def test_tables_are_written_before_another_stream_can_read_them(fake):
+    s = fake.space(6, 7)
+    assert not fake.unfinished(lambda: s.set_integrals(*mc.lieb_integrals(7, 1.0)))
+    fake.L.fake_capture(1)                 # a captured call writes no table that an eager one would read
+    assert packs(fake.kernels(lambda: s.density(1))) == 0
+    fake.L.fake_capture(0)
+    first = fake.kernels(lambda: s.density(1))
+    assert packs(first) == 1
+    s.close()
+    s = fake.space(6, 7)
+    assert s.set_integrals(*mc.lieb_integrals(7, 1.0)) == OK
+    assert packs(fake.unfinished(lambda: s.density(1))) == 0
+    s.close()
