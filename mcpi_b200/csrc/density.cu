@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(DmmaGram<M, SAME>::THREADS, 1)
 // Before, every entry read both its factors from shared memory for each
 // configuration (2 x 16 bytes per 4 multiply-adds, 63 us of shared-memory
 // bandwidth alone at N=16, M=10). Measured with the finish, N=16 and N=20, M=10:
-// 156 -> 60 us and 706 -> 289 us; two states 255 -> 112 us and 1213 -> 562 us.
+// 156 -> 58 us and 706 -> 286 us; two states 255 -> 106 us and 1213 -> 535 us.
 constexpr int kRho1Warps = 8;
 // Up to these M (us at the sizes N, M; this kernel / k_rho1_smem, finish included):
 // one state M=15 N=8 25 / 50, M=16 N=8 45 either way and 27 / 16 at N=6; two
@@ -818,7 +818,7 @@ __device__ __forceinline__ void pair_of(int p, int M, int &k, int &s)
 // entry, its permutations and, where that is not held itself, its conjugate.
 // (One thread per output, adding the partials one after the other, took 41 us
 // after rho1 and 30 us after rho2 at M=10; this takes 3 to 4 us.)
-template <int M, int ORDER, int HERM = 0>
+template <int M, int ORDER, int HERM>
 __global__ void __launch_bounds__(1024) k_gram_finish(const double2 *__restrict__ partial, int nblocks,
                                                       double2 *__restrict__ out)
 {
@@ -862,6 +862,51 @@ __global__ void __launch_bounds__(1024) k_gram_finish(const double2 *__restrict_
     }
 }
 
+// The same for at most eight partials: one thread per output, its partials all in
+// flight and added in the other kernel's order (the same bits), written in runs,
+// where the other one's time is its permuted writes and its blocks of 1,024 threads.
+// Whole calls in us, k_gram_finish / this: rho2 N=2, M=12 15.2 / 13.8, N=2, M=16
+// 20.5 / 16.6, N=4, M=16 (five partials) 22.6 / 20.5; two states N=4, M=15 28.3 /
+// 24.6; up to ten orbitals alike.
+constexpr int kFinishFew = 8;
+
+template <int M, int HERM>
+__global__ void __launch_bounds__(256) k_gram_finish_few(const double2 *__restrict__ partial, int nblocks,
+                                                         double2 *__restrict__ out)
+{
+    using C = Cols<M, 2>;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    if (x >= M * M * M * M) return;
+    const int k = x % M, s = (x / M) % M, q = (x / (M * M)) % M, l = x / (M * M * M);
+    const int a = k <= s ? pair_index(k, s, M) : pair_index(s, k, M);
+    const int b = q <= l ? pair_index(q, l, M) : pair_index(l, q, M);
+    const bool held = gram_held<HERM>(a, b, C::NB);
+    const int e = held ? a * C::K + b : b * C::K + a;
+    double2 p[kFinishFew];
+#pragma unroll
+    for (int blk = 0; blk < kFinishFew; ++blk)
+        p[blk] = blk < nblocks ? partial[(size_t)blk * C::K * C::K + e] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int o = kFinishFew / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) {
+            p[i].x += p[i + o].x;
+            p[i].y += p[i + o].y;
+        }
+    out[x] = held ? p[0] : make_double2(p[0].x, -p[0].y);
+}
+
+template <int M, int ORDER, int HERM>
+cudaError_t gram_finish(const double2 *partial, int nblocks, double2 *out, cudaStream_t st)
+{
+    if constexpr (ORDER == 2)
+        if (nblocks <= kFinishFew)
+            return launch_pdl(k_gram_finish_few<M, HERM>, (M * M * M * M + 255) / 256, 256, 0, st, partial, nblocks, out);
+    constexpr unsigned grid = (Cols<M, ORDER>::K * Cols<M, ORDER>::K + 31) / 32;
+    return launch_pdl(k_gram_finish<M, ORDER, HERM>, grid, 1024, 0, st, partial, nblocks, out);
+}
+
 template <int M, int ORDER>
 cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi,
                       const double2 *psi, double2 *partial, double2 *out, cudaStream_t st, int *status,
@@ -869,7 +914,6 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
 {
     using C = Cols<M, ORDER>;
     const bool same = (phi == psi);
-    constexpr unsigned finish = (C::K * C::K + 31) / 32;
     if constexpr (ORDER == 1) {
         const size_t tab = sizeof(double) * sp.wstride + sizeof(uint32_t) * (M - 1) * sp.wstride;
         auto run = [&](auto state) -> cudaError_t {
@@ -880,7 +924,7 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
                 const unsigned gx = need < (unsigned)kDmmaBlocks ? (need ? need : 1) : kDmmaBlocks;
                 cudaError_t e = launch_pdl(k_rho1<M, SAME>, gx, kRho1Warps * 32, tab, st, sp, tb, phi, psi, partial);
                 if (e != cudaSuccess) return e;
-                return launch_pdl(k_gram_finish<M, 1, SAME ? 3 : 0>, finish, 1024, 0, st, partial, (int)gx, out);
+                return gram_finish<M, 1, SAME ? 3 : 0>(partial, (int)gx, out, st);
             } else {
                 const size_t smem = sizeof(double2) * ((SAME ? 1 : 2) * (size_t)M * (kTile1 + 1) + kThreads) + tab;
                 const unsigned ntiles = (sp.nc1 + kTile1 - 1) / kTile1;
@@ -890,7 +934,7 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
                 if (e != cudaSuccess) return e;
                 k_rho1_smem<M, SAME><<<gx, kThreads, smem, st>>>(sp, tb, phi, psi, partial);
                 if (const cudaError_t le = cudaGetLastError(); le != cudaSuccess) return le;
-                return launch_pdl(k_gram_finish<M, 1, SAME ? 3 : 0>, finish, 1024, 0, st, partial, (int)gx, out);
+                return gram_finish<M, 1, SAME ? 3 : 0>(partial, (int)gx, out, st);
             }
         };
         const cudaError_t e = same ? run(std::true_type{}) : run(std::false_type{});
@@ -914,7 +958,7 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
             e = launch_pdl(k_gram_dmma<M, true>, gx, Dm::THREADS, sm, st, sp, tb, phi, psi, partial, status, wait_cycles,
                            test_stall);
             if (e != cudaSuccess) return e;
-            return launch_pdl(k_gram_finish<M, 2, 2>, finish, 1024, 0, st, partial, (int)gx, out);
+            return gram_finish<M, 2, 2>(partial, (int)gx, out, st);
         }
         if constexpr (M <= kDmmaMaxMTrans) {
             if (!same && DmmaGram<M, false>::smem(sp.wstride) <= (size_t)optin) {
@@ -927,7 +971,7 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
             e = launch_pdl(k_gram_dmma<M, false>, gx, Dm::THREADS, sm, st, sp, tb, phi, psi, partial, status, wait_cycles,
                            test_stall);
             if (e != cudaSuccess) return e;
-            return launch_pdl(k_gram_finish<M, 2, 0>, finish, 1024, 0, st, partial, (int)gx, out);
+            return gram_finish<M, 2, 0>(partial, (int)gx, out, st);
             }
         }
     }
@@ -951,8 +995,8 @@ cudaError_t density_m(const Space &sp, const SpaceTables &tb, const double2 *phi
     }
     // the finish reports its own launch only: without the partials it must not run
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (same) return launch_pdl(k_gram_finish<M, ORDER, 1>, finish, 1024, 0, st, partial, (int)gx, out);
-    return launch_pdl(k_gram_finish<M, ORDER, 0>, finish, 1024, 0, st, partial, (int)gx, out);
+    if (same) return gram_finish<M, ORDER, 1>(partial, (int)gx, out, st);
+    return gram_finish<M, ORDER, 0>(partial, (int)gx, out, st);
 }
 
 }  // namespace
