@@ -22,7 +22,7 @@ def finite_range(M, g):
     return Ho, np.where(k + s == q + l, 0.5 * g * (v(k - l) + v(k - q)), 0.0).reshape(-1).astype(np.complex128)
 
 
-CASES = [(N, M, kind) for N, M in [(256, 2), (257, 2), (258, 2), (300, 2), (600, 2), (260, 3)]
+CASES = [(N, M, kind) for N, M in [(300, 1), (256, 2), (257, 2), (258, 2), (300, 2), (600, 2), (260, 3)]
          for kind in ("lieb", "range", "random")] + [(258, 4, "lieb")]
 
 
