@@ -1237,9 +1237,9 @@ cudaError_t direct_apply_m(const Space &sp, const SpaceTables &tb, const PairOp 
 // kernel 2 gathers one sum per occupied pair of a row. Against the 60 % of
 // predicated-off products of the direct form, that is 90 M gathers of 16 bytes
 // at N=16, M=10 instead of 114 M, and a third of the instructions. Both are
-// bound by the L1 data pipe (72 % and 66 % of peak: consecutive rows gather in
+// bound by the L1 data pipe (71 % and 67 % of peak: consecutive rows gather in
 // short unaligned runs, 8 wavefronts per full request), kernel 2 by issue too
-// (61 %); DRAM carries 0.6 GB. 78 + 133 us at N=16, M=10. Blocks per SM: kernel 1
+// (60 %); DRAM carries 0.6 GB. 76 + 133 us at N=16, M=10. Blocks per SM: kernel 1
 // three (80 registers; four spill: 35 against 31 us at N=12, M=11), kernel 2
 // four up to ten orbitals and three above (N=9, M=13 35 -> 32 us).
 // ---------------------------------------------------------------------------
@@ -1452,10 +1452,13 @@ bool contact_pays(const Space &sp)
 {
     if (!direct_covers(sp)) return true;   // stands in for the two pair kernels
     // against the direct form, measured in us (contact / direct) on rotating
-    // states: M=11 N=10 33 / 35, N=12 69 / 95, N=16 582 / 750; M=10 N=11 28 / 25,
-    // N=12 37 / 37, N=13 58 / 74, N=16 204 / 225, N=18 475 / 512, N=20 1142 / 1118
-    // (its S, 1.4 GB, and the states then leave each other nothing in L2); M=9
-    // N=16 70 / 65, N=20 294 / 274
+    // states. M=11: N=8 13.1 / 13.0, N=9 15.8 / 18.1, N=10 24.5 / 32.2, N=11 38.2 /
+    // 55.2. M=10: N=9 12.1 / 10.1, N=10 13.3 / 14.1, N=11 21.1 / 22.1, N=12 29.0 /
+    // 35.2, N=13 46.6 / 71.1, N=16 205 / 225, N=18 473 / 509, N=19 732 / 758, N=20
+    // 1118 / 1115 (its S, 1.4 GB, and the states then leave each other nothing in
+    // L2). M=9: N=10 11.3 / 8.3, N=14 32.0 / 30.9, N=16 66.8 / 65.0. So M=11 from
+    // N=10 and M=10 from N=12 to 18; the sizes next to these gain 3 to 15 % and keep
+    // the form that needs no intermediate
     return sp.M == 11 ? sp.nc >= 180000 : sp.M == 10 && sp.nc >= 290000 && sp.nc <= 6000000;
 }
 

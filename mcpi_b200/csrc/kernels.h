@@ -18,10 +18,11 @@ namespace mcpi {
 // blocks as they exit, not by an explicit trigger: triggered early, whole
 // chains of waiting kernels became resident and took the slots that spread the
 // next one over the SMs (Lanczos N=10, M=9: 7.8 ms without, 10.0 ms triggered
-// at entry, 5.8 ms after the wait, 5.4 ms at exit). Measured (B200): H.psi
-// N=9, M=13 49.8 -> 44.2 us, N=16, M=10 209 -> 198 us, general N=10, M=10 38.9 ->
-// 34.7 us; H.psi, its adjoint and both transition densities at N=8, M=8 59.6 ->
-// 52.5 us; 100 Lanczos steps N=12, M=8 8.0 -> 5.8 ms.
+// at entry, 5.8 ms after the wait, 5.4 ms at exit). Measured (B200; the same
+// kernels launched without / with it): H.psi N=9, M=13 47.0 / 42.4 us, N=16, M=10
+// 203.6 / 197.0 us, general N=10, M=10 38.9 / 34.7 us; H.psi, its adjoint and both
+// transition densities at N=8, M=8 57.2 / 49.4 us; 100 Lanczos steps N=12, M=8
+// 5.25 / 3.51 ms, N=10, M=9 5.32 / 3.44 ms.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 

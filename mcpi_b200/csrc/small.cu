@@ -2,10 +2,9 @@
 //
 // The launch sequence of lanczos.cu takes eight kernels per step. On a space of
 // a few thousand configurations they leave the chip idle: at N=5, M=11 (3,003
-// rows) 3 blocks form the basis' dot products and 12 the update, each thread a
-// serial chain over up to 375 basis vectors, about 120 us per step. Here the
-// whole solve is one cooperative launch over all SMs with three grid barriers
-// per step:
+// rows) 12 blocks do the update, each thread a serial chain over up to 375 basis
+// vectors, and a step's 34 us are mostly launches and latency. Here the whole
+// solve is one cooperative launch over all SMs with three grid barriers per step:
 //   1. v_{i+1} = r / beta (whole, in every block's shared memory), and by rows
 //      w = H v_{i+1} - beta v_i with the shares of alpha;
 //   2. x = w - alpha v_{i+1} (whole, in shared memory), and one warp per
@@ -24,7 +23,8 @@
 // groups), each with the coefficients and columns of its block's terms, built
 // once at the start of each solve and read from L2 (a few MB).
 //
-// Measured (B200, N=5, M=11, 375 steps, whole mcpi_ground): 54.0 -> 12.5 ms.
+// Measured (B200, N=5, M=11, 375 steps, whole mcpi_ground, of which 6.5 ms are the
+// host's tridiagonal): 19.8 -> 12.8 ms.
 // Barrier waits are bounded (about two seconds, then the status word reports
 // MCPI_ERR_TIMEOUT and every block leaves at its next barrier).
 #include <cuda_runtime.h>
@@ -224,7 +224,7 @@ __device__ __forceinline__ bool grid_barrier(const SmallArgs &a, unsigned k)
 
 // Sum of 32-row shares in the order of the launch sequence: eight shares to a
 // 256-row block, thread b < 256 of the final sum takes block b, its warps are
-// added in order. At most 64 blocks. One warp; the result is in lane 0.
+// added in order (kSmallMaxRows: 22 blocks). One warp; the result is in lane 0.
 template <class Load>
 __device__ __forceinline__ double2 sum_shares(uint32_t nshares, Load load)
 {
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kST, 1) k_small_lanczos(SmallArgs a)
         if (nvec && !grid_barrier(a, nbar++)) return;
         // 3. rows: r = x - sum_j c_j V_j, shares of |r|^2
         for (int j = threadIdx.x; j < nvec; j += kST) {
-            // the warp sum of k_multidot_finish over the slices (at most 16)
+            // the warp sum of k_multidot_finish over the slices (six at most)
             double2 p[16];
 #pragma unroll
             for (int s = 0; s < 16; ++s)
