@@ -197,8 +197,11 @@ def _torch():
     return torch
 
 
-# per thread: whether row ranges belong to a sharded solve (distributed.solve_rows)
-_rows = threading.local()
+class _Rows(threading.local):
+    solve = False   # whether this thread's row ranges belong to a sharded solve (distributed.solve_rows)
+
+
+_rows = _Rows()
 
 
 class FockSpace:
@@ -340,7 +343,7 @@ class FockSpace:
         C = self._vec(C)
         out = self.empty(row1 - row0) if out is None else out
         self._stream()
-        f = lib().mcpi_shard_apply_h if getattr(_rows, "solve", False) else lib().mcpi_apply_h_rows
+        f = lib().mcpi_shard_apply_h if _rows.solve else lib().mcpi_apply_h_rows
         _check(f(self._h, _vp(C.data_ptr()), row0, row1, _vp(out.data_ptr()) if row1 > row0 else None))
         return out
 

@@ -559,7 +559,7 @@ int ensure_gram(mcpi_space_s *sp)
 
 int apply_op(mcpi_space_s *sp, const DevPairOp &op, const void *d_C, void *d_out)
 {
-    CHECK_ARG(sp && d_C && d_out, "null argument");
+    CHECK_ARG(d_C && d_out, "null argument");
     if (!sp->has_op) return fail(MCPI_ERR_STATE, "mcpi_set_integrals has not been called");
     CHECK_ARG(d_C != d_out, "input and output must not alias");
     DeviceGuard g(sp->device);
@@ -1058,7 +1058,11 @@ int mcpi_set_integrals(mcpi_space sp, const double *h_Ho, const double *h_Hint, 
     return MCPI_OK;
 }
 
-int mcpi_apply_h(mcpi_space sp, const void *d_C, void *d_out) { return apply_op(sp, sp ? sp->fwd : DevPairOp{}, d_C, d_out); }
+int mcpi_apply_h(mcpi_space sp, const void *d_C, void *d_out)
+{
+    CHECK_ARG(sp, "null argument");
+    return apply_op(sp, sp->fwd, d_C, d_out);
+}
 
 int mcpi_apply_h_host(mcpi_space sp, int count, const void *const *h_C, void *const *h_out)
 {
@@ -1203,7 +1207,8 @@ int mcpi_shard_apply_h(mcpi_space sp, const void *d_C, int64_t row0, int64_t row
 
 int mcpi_apply_h_adjoint(mcpi_space sp, const void *d_C, void *d_out)
 {
-    return apply_op(sp, sp ? sp->adj : DevPairOp{}, d_C, d_out);
+    CHECK_ARG(sp, "null argument");
+    return apply_op(sp, sp->adj, d_C, d_out);
 }
 
 static int density(mcpi_space sp, int order, const void *phi, const void *psi, void *out)

@@ -50,7 +50,7 @@ def solve_rows():
     one (contact interactions of an odd number of plane waves), and there the
     recurrence amplifies rounding to order one. ShardedLanczos applies its local
     operator inside."""
-    before = getattr(_rows, "solve", False)
+    before = _rows.solve
     _rows.solve = True
     try:
         yield

@@ -307,3 +307,26 @@ def test_tables_are_written_before_another_stream_can_read_them(fake):
     assert s.set_integrals(*mc.lieb_integrals(7, 1.0)) == OK
     assert packs(fake.unfinished(lambda: s.density(1))) == 0
     s.close()
+
+
+def test_calls_without_pool_memory_take_the_direct_form(fake):
+    s = fake.space(12, 10)
+    assert s.set_integrals(*mc.lieb_integrals(10, 1.0)) == OK
+    for call in (s.apply_h, s.apply_h_adjoint, lambda: s.rows(0, s.nc)):
+        for got, refused in (("contact", False), ("direct", True), ("contact", False)):
+            fake.L.fake_fail_pool(0 if refused else -1, 0)
+            assert forms(fake.kernels(call)) == {got}
+    t = fake.space(13, 10)
+    fake.L.fake_headroom(1 << 20)          # its S takes 51 MB, the pool holds 28
+    assert t.set_integrals(*mc.lieb_integrals(10, 1.0)) == OK
+    assert forms(fake.kernels(t.apply_h)) == {"direct"}
+    t.close()
+    s.close()
+
+
+@pytest.mark.parametrize("N,form", [(18, "contact"), (19, "direct")])
+def test_the_contact_scratch_is_at_most_2_gib(fake, N, form):
+    s = fake.space(N, 11)                  # S of 1.8 and 2.8 GB
+    assert s.set_integrals(*mc.lieb_integrals(11, 1.0)) == OK
+    assert forms(fake.kernels(s.apply_h)) == {form}
+    s.close()
