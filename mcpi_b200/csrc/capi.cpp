@@ -233,13 +233,19 @@ std::vector<double> pack_contact(const std::vector<cplx> &Ht, int P, int M)
     return f;
 }
 
+// Host arrays of an operator on their way to the device, until the stream is synchronised.
+struct OpArrays {
+    std::vector<int> rowptr, prog;
+    std::vector<uint16_t> col;
+    std::vector<cplx> val, mom;
+};
+
 int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, const cplx *hdiag,
-              const cplx *hfull)
+              const cplx *hfull, OpArrays &host)
 {
     const int P = sp->P, M = sp->M;
-    std::vector<int> rowptr(P + 1, 0);
-    std::vector<uint16_t> col;
-    std::vector<cplx> val;
+    auto &[rowptr, prog, col, val, mom] = host;
+    rowptr.assign(P + 1, 0);
     for (int a = 0; a < P; ++a) {
         for (int b = 0; b < P; ++b) {
             const cplx h = Ht[(size_t)a * P + b];
@@ -264,7 +270,7 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
     }
     CK(cudaMemcpyAsync(op.hdiag, hdiag, sizeof(double2) * M, cudaMemcpyHostToDevice, sp->stream));
     CK(cudaMemcpyAsync(op.hfull, hfull, sizeof(double2) * M * M, cudaMemcpyHostToDevice, sp->stream));
-    const std::vector<cplx> mom = pack_momentum(Ht, P, M);
+    mom = pack_momentum(Ht, P, M);
     if (!mom.empty() && !sp->dense_only && sp->kernel_choice != 2) {
         CK(dev_malloc(sp, &op.hblk, sizeof(double2) * mom.size()));
         CK(cudaMemcpyAsync(op.hblk, mom.data(), sizeof(double2) * mom.size(), cudaMemcpyHostToDevice, sp->stream));
@@ -276,7 +282,7 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
         for (const cplx &h : mom) op.real = op.real && h.imag() == 0.0;
         for (int k = 0; k < M; ++k) op.real = op.real && hdiag[k].imag() == 0.0;
     }
-    const std::vector<int> prog = pack_blocks(Ht, P, M);
+    prog = pack_blocks(Ht, P, M);
     if (!prog.empty() && !sp->dense_only) {
         CK(dev_malloc(sp, &op.prog, sizeof(int) * prog.size()));
         CK(cudaMemcpyAsync(op.prog, prog.data(), sizeof(int) * prog.size(), cudaMemcpyHostToDevice, sp->stream));
@@ -290,7 +296,6 @@ int upload_op(mcpi_space_s *sp, DevPairOp &op, const std::vector<cplx> &Ht, cons
         CK(dev_malloc(sp, &op.hdense, sizeof(double2) * P * P));
         CK(cudaMemcpyAsync(op.hdense, Ht.data(), sizeof(double2) * P * P, cudaMemcpyHostToDevice, sp->stream));
     }
-    CK(cudaStreamSynchronize(sp->stream));  // host vectors go out of scope
     op.nnz = (int)col.size();
     return MCPI_OK;
 }
@@ -1016,10 +1021,13 @@ int mcpi_set_integrals(mcpi_space sp, const double *h_Ho, const double *h_Hint, 
     std::vector<cplx> Hta((size_t)P * P);
     for (int a = 0; a < P; ++a)
         for (int b = 0; b < P; ++b) Hta[(size_t)b * P + a] = std::conj(Ht[(size_t)a * P + b]);
-    int rc = upload_op(sp, sp->fwd, Ht, hd.data(), hf.data());
-    if (rc) return rc;
-    rc = upload_op(sp, sp->adj, Hta, hda.data(), hfa.data());
-    if (rc) return rc;
+    OpArrays fwd, adj;
+    int rc = upload_op(sp, sp->fwd, Ht, hd.data(), hf.data(), fwd);
+    if (rc == MCPI_OK) rc = upload_op(sp, sp->adj, Hta, hda.data(), hfa.data(), adj);
+    if (rc) {
+        cudaStreamSynchronize(sp->stream);   // the host arrays go out of scope
+        return rc;
+    }
     sp->fwd.create_form = sp->adj.create_form = sp->create_form;
     sp->fwd.status = sp->adj.status = sp->d_status;
     sp->fwd.wait_cycles = sp->adj.wait_cycles = sp->wait_cycles;
@@ -1038,9 +1046,8 @@ int mcpi_set_integrals(mcpi_space sp, const double *h_Ho, const double *h_Hint, 
             s2.nc = (uint32_t)sp->nc2;
             cudaError_t e = mcpi::launch_pack_occ(sp->sp, t, sp->d_occ, bits, sp->stream);
             if (e == cudaSuccess) e = mcpi::launch_pack_occ(s2, t, sp->d_occ2, bits, sp->stream);
-            // written before any stream can read them, the space's next one included
-            if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);
-            if (e != cudaSuccess) {   // no table is left that may not have been written
+            if (e != cudaSuccess) {   // no table is left that was not written
+                cudaStreamSynchronize(sp->stream);   // the host arrays go out of scope
                 cudaFree(sp->d_occ);
                 cudaFree(sp->d_occ2);
                 sp->d_occ = sp->d_occ2 = nullptr;
@@ -1054,6 +1061,9 @@ int mcpi_set_integrals(mcpi_space sp, const double *h_Ho, const double *h_Hint, 
             sp->d_occ2 = nullptr;
         }
     }
+    // the host arrays are on the device and the tables written before any stream,
+    // the space's next one included, can read them
+    CK(cudaStreamSynchronize(sp->stream));
     sp->has_op = true;
     return MCPI_OK;
 }
@@ -1229,7 +1239,8 @@ static int density(mcpi_space sp, int order, const void *phi, const void *psi, v
             s1.nc = (uint32_t)sp->nc1;
             cudaError_t e = mcpi::launch_pack_occ(s1, mcpi::SpaceTables{sp->d_W, sp->d_sq}, sp->d_occ1, sp->occ_bits,
                                                   sp->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);   // as above
+            // written before any stream can read it
+            if (e == cudaSuccess) e = cudaStreamSynchronize(sp->stream);
             if (e != cudaSuccess) {
                 cudaFree(sp->d_occ1);
                 sp->d_occ1 = nullptr;
